@@ -60,8 +60,9 @@ __device__ __forceinline__ U4 philox4x32_10_rk(uint32_t c0, uint32_t c1, uint32_
 {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c0, p1 = (uint64_t)0xCD9E8D57u * c2;
+        const uint32_t hi0 = (uint32_t)(p0 >> 32), lo0 = (uint32_t)p0;
+        const uint32_t hi1 = (uint32_t)(p1 >> 32), lo1 = (uint32_t)p1;
         const uint32_t n0 = hi1 ^ c1 ^ rk[2 * r], n2 = hi0 ^ c3 ^ rk[2 * r + 1];
         c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
     }
@@ -106,7 +107,13 @@ template <> struct M<float> {
     __device__ __forceinline__ static float log(float x) { return __logf(x); }
     // -log(u) for u in (0,1), never below 1 - u (> 0): the fast logarithm's
     // absolute error near 1 could otherwise give 0 or a negative value
-    __device__ __forceinline__ static float neglog(float u) { return fmaxf(-__logf(u), 1.f - u); }
+    // (u is never subnormal: the flushing form of the logarithm)
+    __device__ __forceinline__ static float neglog(float u)
+    {
+        float l;
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u));
+        return fmaxf(-(l * 0.693147180559945f), 1.f - u);
+    }
     __device__ __forceinline__ static void sincos(float x, float *s, float *c) { __sincosf(x, s, c); }
     __device__ __forceinline__ static float sqrt(float x) { return sqrtf(x); }
     __device__ __forceinline__ static float acos(float x) { return acosf(x); }

@@ -15,6 +15,7 @@
 #include <curand_philox4x32_x.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "tam_device.cuh"
 #include "tam_kernels.h"
@@ -84,15 +85,26 @@ __device__ __forceinline__ void fetch(const TransportArgs &a, const MatR<Real> *
     }
 }
 
-// Event loop per lane: DEAD (needs a packet) -> FLY (one voxel step per
-// iteration: cross a face, reach an outer face, or reach the interaction
-// point) -> SCAT (waits at the interaction point) or FACE (waits on an outer
-// face for its Fresnel draw) -> FLY ...  The events (Philox block, HG
-// rotation, roulette, new optical depth; Fresnel reflect-or-escape) are the
-// expensive part; the event batch runs once at least scat_min lanes of the
-// warp wait, or when no lane is flying, so it executes with most lanes
-// active.  Every packet sees the same sequence of events and random numbers
-// as a straight loop.
+// A lane is alive (holds a packet) or dead, and while alive its packet either
+// flies on (`go`: its next event is the crossing of a voxel face) or waits for
+// the event batch, at an interaction point or on an outer face.  `go` is
+// worked out ahead, at the end of the step before, so a flight of k crossings
+// takes k steps and a lane that has stopped is left as it is by further steps:
+// the step is straight-line code under one predicate, without branches.  The
+// events (Philox block, HG rotation, roulette, new optical depth; Fresnel
+// reflect-or-escape) are the expensive part; the event batch runs once at
+// least scat_min lanes of the warp wait (in FP32 fewer when lanes are dead, see
+// wait_min), or when no lane flies, so it executes with most lanes active.
+// Every packet sees the same sequence of events and random numbers as a
+// straight loop.
+//
+// What bounds it is instruction issue (80 % of cycles; 23 of 32 lanes active):
+// on the 200^3 bench pass (1e8 packets) this form takes 369 ms against 510 ms
+// for a step that tested the lane's state, the cap and the interaction in
+// nested branches (5491 -> about 3900 warp instructions per packet); 47 against
+// 64 ms per 1e7 packets on the three-layer slab, 154 against 192 ms on a 384^3
+// vessel grid.  scat_min 12 to 24 are within 1 % of each other; 2, 3 and 6
+// voxel steps per vote are 5, 3 and 2 % slower than 4.
 //
 // The DDA is incremental (Amanatides & Woo): per flight, the distance tm to
 // the next face of each axis and the cell width td along the ray; a crossing
@@ -105,9 +117,10 @@ template <typename Real> __device__ __forceinline__ const TrConst<Real> &consts(
 }
 
 template <typename Real, int MED, bool T32>
-__global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) transport_kernel(const __grid_constant__ TransportArgs a, int scat_min)
+__global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) transport_kernel(const __grid_constant__ TransportArgs a, int scat_min, unsigned lanes)
 {
     __shared__ MatR<Real> lut[MAX_MAT];
+    __shared__ HgF hgt[sizeof(Real) == 4 ? MAX_MAT : 1];
     for (int t = threadIdx.x; t < MAX_MAT; t += blockDim.x) {
         const OptMat &o = a.lut[t < a.nmat ? t : 0];
         MatR<Real> m;
@@ -118,6 +131,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
         m.g2 = (Real)(o.g * o.g);
         m.n = (Real)o.n;
         lut[t] = m;
+        if constexpr (sizeof(Real) == 4) hgt[t] = hg_consts(m.g, m.g2);
     }
     // per-packet (rare) tallies accumulate in shared memory, not registers
     __shared__ double s_tal[5];  // specular, reflected, transmitted, side, roulette net
@@ -139,7 +153,9 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     const uint32_t strm = a.stream_dev ? *a.stream_dev : a.stream;
     const unsigned lane = threadIdx.x & 31u;
     const Real wmin = K.wmin, rm = K.rm, inv_rm = K.inv_rm;
-    const int NX = a.nx, NY = a.ny, NZ = a.nz, SY = a.nx, SZ = a.nx * a.ny;
+    // weights below this need a look after a scatter: roulette, or the end of a packet without weight
+    const Real w_rare = a.roulette && wmin > (Real)0 ? wmin : (Real)1.401298464e-45;
+    const int NX = a.nx, NY = a.ny, NZ = a.nz;
     const uint32_t max_steps = a.max_steps > 0xfffffff0ll ? 0xfffffff0u : (uint32_t)a.max_steps;
     const Real namb = K.namb;
     // FP32 in a uniform medium: the flight is tracked by distance (tau / mut
@@ -153,9 +169,10 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     // (config mode's factor is exactly 1)
     constexpr bool NUDGE = MED == MED_RHOKAP;
 
-    int mode = M_DEAD;
+    bool alive = false;
     bool exhausted = false;
-    int ix = 0, iy = 0, iz = 0, cidx = 0, mid = 0, sgx = 1, sgy = 1, sgz = 1, fax = 0;
+    int ix = 0, iy = 0, iz = 0, mid = 0, sgx = 1, sgy = 1, sgz = 1;
+    auto cell = [&]() { return ix + NX * (iy + NY * iz); };
     Real fx = 0, fy = 0, fz = 0, nx = 0, ny = 0, nz = 0, sint = 0, phi = 0;
     Real cpv = 1, spv = 0;  // FP32 path: (cos phi, sin phi) in place of phi
     Real tdx = 0, tdy = 0, tdz = 0, tmx = 0, tmy = 0, tmz = 0, t = 0;
@@ -169,21 +186,22 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
             mut = mut_u;
             mua = mua_u;
         } else {
-            fetch<Real, MED>(a, lut, ix, iy, iz, cidx, mut, mua, mid);
+            fetch<Real, MED>(a, lut, ix, iy, iz, cell(), mut, mua, mid);
         }
     };
 
     for (;;) {
         // ---------------------------------------------- refill dead lanes --
         // (exhausted is warp-uniform: set once the counter has passed n)
-        const unsigned need = exhausted ? 0u : __ballot_sync(FULL, mode == M_DEAD);
-        if (need && (__popc(need) >= TAM_REFILL_MIN || need == FULL)) {
+        unsigned live = __ballot_sync(FULL, alive);
+        const unsigned need = exhausted ? 0u : ~live & lanes;
+        if (need && (__popc(need) >= TAM_REFILL_MIN || live == 0u)) {
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if ((int)lane == leader) base = atomicAdd(a.work, (unsigned long long)__popc(need));
             base = __shfl_sync(FULL, base, leader);
             exhausted = base + (unsigned long long)__popc(need) >= (unsigned long long)a.n;
-            if (mode == M_DEAD) {
+            if (need >> lane & 1u) {
                 const unsigned long long my = base + __popc(need & ((1u << lane) - 1u));
                 if (my < (unsigned long long)a.n) {
                     // launch (src/sourceph.f90:7-49; Gaussian beam in config mode)
@@ -223,7 +241,6 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                         ix = ix > NX - 1 ? NX - 1 : ix;
                         iy = iy > NY - 1 ? NY - 1 : iy;
                         iz = NZ - 1;
-                        cidx = ix + SY * iy + SZ * iz;
                         fx = X - (Real)ix * hx;
                         fy = Y - (Real)iy * hy;
                         fz = hz - (Real)1.e-8 * hz;
@@ -247,214 +264,267 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                         t = (Real)0;
                         dep = (Real)0;
                         nsteps = 0;
-                        mode = M_FLY;
+                        alive = true;
                     }
                 }
             }
+            live = __ballot_sync(FULL, alive);
         }
-        // ------------------------------------------------- flight phase --
-        // voxel steps of the flying lanes until enough lanes wait to scatter,
-        // no lane flies, or a lane needs a new packet
-        unsigned sc, fl;
-        // -------------------------- one voxel step (src/inttau2.f90:37-63) --
-        auto vstep = [&]() {
-        if (mode == M_FLY) {
-            if (++nsteps > max_steps) {
-                if (dep != (Real)0) deposit<T32>(a, cidx, ix, iy, iz, dep);
-                dep = (Real)0;
-                atomicAdd(a.tally + T_OVERFLOW, 1.0);
-                atomicOr(&s_err, (unsigned)DEVERR_STEP_CAP);
-                cSteps += nsteps;
-                mode = M_DEAD;
-            } else {
-                // nearest face; ties go z over y over x (src/inttau2.f90:116-118)
-                int ax = 2;
-                Real tmin = tmz;
-                if (tmy < tmin) { tmin = tmy; ax = 1; }
-                if (tmx < tmin) { tmin = tmx; ax = 0; }
-                Real dw;
-                bool cross;
-                if constexpr (DIST) {
-                    // tau holds the flight distance of the interaction point
-                    cross = tmin < tau;
-                    const Real tend = cross ? tmin : tau;
-                    dw = tend - t;
-                    dw = dw < (Real)0 ? (Real)0 : dw;
-                    dep += w * dw * mua;
-                    t = tend;
-                } else {
-                    dw = tmin - t;
-                    dw = dw < (Real)0 ? (Real)0 : dw;
-                    const Real taucell = dw * mut;
-                    cross = taucell < tau;
-                    if (cross) {
-                        dep += w * dw * mua;
-                        tau -= taucell;
-                        t = tmin;
-                    }
-                }
-                if (cross) {
-                    const bool cx = ax == 0, cy = ax == 1, cz = ax == 2;
-                    const int sg = cx ? sgx : (cy ? sgy : sgz);
-                    const int j = (cx ? ix : (cy ? iy : iz)) + sg;
-                    const int N = cx ? NX : (cy ? NY : NZ);
-                    deposit<T32>(a, cidx, ix, iy, iz, dep);
-                    dep = (Real)0;
-                    if ((unsigned)j < (unsigned)N) {
-                        // step into the next cell (branch-free over the axis); the
-                        // reference snaps the crossed coordinate to the face +- delta
-                        // (src/inttau2.f90:140-169), which knx/kny/knz carry
-                        ix = cx ? j : ix;
-                        iy = cy ? j : iy;
-                        iz = cz ? j : iz;
-                        cidx += cx ? sg : (cy ? sg * SY : sg * SZ);
-                        tmx = cx ? tmx + (NUDGE ? tdx * knx : tdx) : tmx;
-                        tmy = cy ? tmy + (NUDGE ? tdy * kny : tdy) : tmy;
-                        tmz = cz ? tmz + (NUDGE ? tdz * knz : tdz) : tmz;
-                        props();
-                    } else if (a.fresnel) {
-                        // outer face: the packet sits on it; the Fresnel draw
-                        // waits for the event batch
-                        fax = ax;
-                        mode = M_FACE;
-                    } else {
-                        // outer face without Fresnel: escape
-                        atomicAdd(&s_tal[cz ? (sgz > 0 ? 1 : 2) : 3], (double)w);
-                        cSteps += nsteps;
-                        mode = M_DEAD;
-                    }
-                } else {
-                    // interaction point inside this cell; the in-cell position
-                    // is reconstructed in the event batch
-                    if constexpr (!DIST) {
-                        const Real dd = M<Real>::div(tau, mut);
-                        dep += w * dd * mua;
-                        t += dd;
-                    }
-                    mode = M_SCAT;
-                }
-            }
-        }
-        };
-        for (;;) {
-            // TAM_VSTEPS voxel steps per vote (transport_common.cuh)
-#pragma unroll
-            for (int q = 0; q < TAM_VSTEPS; ++q) vstep();
-            sc = __ballot_sync(FULL, mode >= M_SCAT);
-            fl = __ballot_sync(FULL, mode == M_FLY);
-            if (fl == 0 || __popc(sc) >= scat_min || (!exhausted && __popc(~(sc | fl)) >= TAM_REFILL_MIN)) break;
-        }
-        if ((sc | fl) == 0) {
+        if (live == 0u) {
             if (exhausted) break;
             continue;
+        }
+        // ------------------------------------------------- flight phase --
+        // voxel steps of the flying lanes until enough lanes wait for the
+        // event batch or none flies
+        Real tmin, ahead;
+        bool px = false, py = false, pz = false;  // FP64: the axis of the next face
+        // whether the flight's interaction point lies beyond the next face
+        // (ties between faces go z over y over x, src/inttau2.f90:116-118)
+        auto look = [&]() {
+            if constexpr (sizeof(Real) == 4) {
+                tmin = fminf(fminf(tmx, tmy), tmz);
+            } else {
+                const bool yz = less_pos(tmy, tmz);
+                tmin = yz ? tmy : tmz;
+                px = less_pos(tmx, tmin);
+                tmin = px ? tmx : tmin;
+                py = yz && !px;
+                pz = !yz && !px;
+            }
+            ahead = DIST ? tmin : (tmin - t) * mut;  // distance, or optical depth to the face
+            return less_pos(ahead, tau);
+        };
+        bool go = look() && alive, capped = false;
+        // one voxel step (src/inttau2.f90:37-63) of the lanes with `go`
+        auto vstep = [&](auto careful) {
+            if constexpr (decltype(careful)::value) {
+                // a packet past its step cap ends here, before the step
+                if (go && nsteps >= max_steps) {
+                    nsteps += 1;
+                    capped = true;
+                    go = false;
+                }
+            }
+            const Real d = dep + w * (tmin - t) * mua;
+            if (go) deposit<T32>(a, cell(), ix, iy, iz, d);
+            // step into the next cell, branch-free over the axis; the
+            // reference snaps the crossed coordinate to the face +- delta
+            // (src/inttau2.f90:140-169), which knx/kny/knz carry.  Past an
+            // outer face the lane waits for the event batch.
+            if constexpr (sizeof(Real) == 4) {
+                int g = go;
+                fly_cross(tmx, tmy, tmz, t, dep, tmin, tau, ix, iy, iz, nsteps, g, NUDGE ? tdx * knx : tdx,
+                          NUDGE ? tdy * kny : tdy, NUDGE ? tdz * knz : tdz, DIST ? 0.f : ahead, sgx, sgy, sgz, NX, NY, NZ);
+                go = g != 0;
+            } else {
+                nsteps += go ? 1u : 0u;
+                dep = go ? (Real)0 : dep;
+                tau = go ? tau - ahead : tau;
+                t = go ? tmin : t;
+                const bool cx = go && px, cy = go && py, cz = go && pz;
+                tmx = cx ? tmx + (NUDGE ? tdx * knx : tdx) : tmx;
+                tmy = cy ? tmy + (NUDGE ? tdy * kny : tdy) : tmy;
+                tmz = cz ? tmz + (NUDGE ? tdz * knz : tdz) : tmz;
+                ix += cx ? sgx : 0;
+                iy += cy ? sgy : 0;
+                iz += cz ? sgz : 0;
+                go = go && (unsigned)ix < (unsigned)NX && (unsigned)iy < (unsigned)NY && (unsigned)iz < (unsigned)NZ;
+            }
+            if constexpr (MED != MED_UNIFORM) {
+                if (go) props();
+            }
+            go = look() && go;
+        };
+        {
+            const int thr = sizeof(Real) == 4 ? wait_min(scat_min, __popc(live)) : scat_min;
+            // a flight crosses at most NX + NY + NZ faces between two outer
+            // faces, so only packets that near their cap need the test per step
+            const uint32_t far = (uint32_t)NX + (uint32_t)NY + (uint32_t)NZ + 2u;
+            if (max_steps >= far && !__any_sync(FULL, alive && nsteps > max_steps - far)) {
+                for (;;) {
+                    const unsigned fl = __ballot_sync(FULL, go);
+                    if (fl == 0u || __popc(live & ~fl) >= thr) break;
+                    if constexpr (DIST && !T32) {
+                        int g = go;
+                        fly_steps(tmx, tmy, tmz, t, dep, tmin, ix, iy, iz, nsteps, g, tdx, tdy, tdz, w, mua, tau, sgx, sgy,
+                                  sgz, NX, NY, NZ, a.jmean);
+                        go = g != 0;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < VSTEPS; ++q) vstep(std::false_type{});
+                    }
+                }
+            } else {
+                for (;;) {
+                    const unsigned fl = __ballot_sync(FULL, go);
+                    if (fl == 0u || __popc(live & ~fl) >= thr) break;
+                    vstep(std::true_type{});
+                }
+                // the interaction counts as a step too
+                const bool in = (unsigned)ix < (unsigned)NX && (unsigned)iy < (unsigned)NY && (unsigned)iz < (unsigned)NZ;
+                if (alive && !go && !capped && in && nsteps >= max_steps) {
+                    nsteps += 1;
+                    capped = true;
+                }
+                if (capped) {
+                    if (dep != (Real)0) deposit<T32>(a, cell(), ix, iy, iz, dep);
+                    dep = (Real)0;
+                    atomicAdd(a.tally + T_OVERFLOW, 1.0);
+                    atomicOr(&s_err, (unsigned)DEVERR_STEP_CAP);
+                    cSteps += nsteps;
+                    alive = false;
+                }
+            }
         }
 
         // ------------------------------------------------- event batch --
         // interactions (implicit capture, HG scatter, roulette) and Fresnel
         // faces, handled together once enough lanes wait; both kinds draw
         // their uniforms from one Philox block per lane
-        if (sc && (__popc(sc) >= scat_min || fl == 0)) {
-            if (mode >= M_SCAT) {
-                const bool face = mode == M_FACE;
-                if (!face) w *= MED == MED_RHOKAP ? (Real)0 : lut[mid].alb;
-                bool die = !face && !(w > (Real)0);
-                U4 r{0u, 0u, 0u, 0u};
-                if (!die) r = philox4x32_10_rk(ev++, plo, phi32, strm, a.rk);
-                if (face) {
-                    const bool cx = fax == 0, cy = fax == 1;
-                    const Real nc = cx ? nx : (cy ? ny : nz);
-                    const Real nt = MED == MED_RHOKAP ? K.rhokap_n : lut[mid].n;
-                    if (Uniform<Real>::from(r.x) < fresnel<Real>(nt, namb, M<Real>::abs(nc))) {
-                        // reflect: mirror the crossed direction component; the
-                        // next face along it is one cell width back
-                        if (cx) {
-                            fy = axis_pos(ny, fy, hy, tmy, t);
-                            fz = axis_pos(nz, fz, hz, tmz, t);
-                            fx = sgx > 0 ? hx : (Real)0;
-                            nx = -nx;
-                            sgx = -sgx;
-                            tmx = t + tdx;
-                            if constexpr (sizeof(Real) == 4) {
-                                cpv = -cpv;  // phi -> PI - phi
-                            } else {
-                                phi = (Real)PI_R - phi;
-                                if (phi < (Real)0) phi += TWOPI;
-                            }
-                        } else if (cy) {
-                            fx = axis_pos(nx, fx, hx, tmx, t);
-                            fz = axis_pos(nz, fz, hz, tmz, t);
-                            fy = sgy > 0 ? hy : (Real)0;
-                            ny = -ny;
-                            sgy = -sgy;
-                            tmy = t + tdy;
-                            if constexpr (sizeof(Real) == 4) {
-                                spv = -spv;  // phi -> TWOPI - phi
-                            } else {
-                                phi = TWOPI - phi;
-                            }
-                        } else {
-                            fx = axis_pos(nx, fx, hx, tmx, t);
-                            fy = axis_pos(ny, fy, hy, tmy, t);
-                            fz = sgz > 0 ? hz : (Real)0;
-                            nz = -nz;
-                            sgz = -sgz;
-                            tmz = t + tdz;
-                        }
-                        mode = M_FLY;
-                    } else {
-                        atomicAdd(&s_tal[(!cx && !cy) ? (sgz > 0 ? 1 : 2) : 3], (double)w);
-                        cSteps += nsteps;
-                        mode = M_DEAD;
-                    }
-                } else if (!die) {
-                    cScat += 1;
-                    fx = axis_pos(nx, fx, hx, tmx, t);
+        {
+            const bool cx = (unsigned)ix >= (unsigned)NX, cy = (unsigned)iy >= (unsigned)NY;
+            const bool cz = (unsigned)iz >= (unsigned)NZ, face = cx || cy || cz;
+            // the packet's end
+            auto end = [&]() {
+                if (dep != (Real)0) deposit<T32>(a, cell(), ix, iy, iz, dep);
+                dep = (Real)0;
+                cSteps += nsteps;
+                alive = false;
+            };
+            // on to the interaction point inside this cell
+            auto interact = [&]() {
+                nsteps += 1;
+                if constexpr (DIST) {
+                    // tau holds the flight distance of the interaction point
+                    dep += w * (tau - t) * mua;
+                    t = tau;
+                } else {
+                    const Real dd = M<Real>::div(tau, mut);
+                    dep += w * dd * mua;
+                    t += dd;
+                }
+                w *= MED == MED_RHOKAP ? (Real)0 : lut[mid].alb;
+            };
+            // an outer face: reflect or escape (without Fresnel: escape)
+            auto surface = [&](uint32_t draw) {
+                const Real nc = cx ? nx : (cy ? ny : nz);
+                const Real nt = MED == MED_RHOKAP ? K.rhokap_n : lut[mid].n;
+                if (!a.fresnel || !(Uniform<Real>::from(draw) < fresnel<Real>(nt, namb, M<Real>::abs(nc)))) {
+                    atomicAdd(&s_tal[cz ? (sgz > 0 ? 1 : 2) : 3], (double)w);
+                    cSteps += nsteps;  // nothing to deposit: the crossing did
+                    alive = false;
+                    return;
+                }
+                // reflect, back into the cell it came from: mirror the crossed
+                // direction component; the next face along it is one cell
+                // width back
+                if (cx) {
+                    ix -= sgx;
                     fy = axis_pos(ny, fy, hy, tmy, t);
                     fz = axis_pos(nz, fz, hz, tmz, t);
-                    Real cost = nz;
+                    fx = sgx > 0 ? hx : (Real)0;
+                    nx = -nx;
+                    sgx = -sgx;
+                    tmx = t + tdx;
                     if constexpr (sizeof(Real) == 4) {
-                        if (stokes_f32(lut[mid].g, lut[mid].g2, Uniform<Real>::from(r.x), Uniform<Real>::from(r.y), cost,
-                                       sint, cpv, spv)) {
-                            nx = sint * cpv;
-                            ny = sint * spv;
-                            nz = cost;
-                        }
+                        cpv = -cpv;  // phi -> PI - phi
                     } else {
-                        Real cp, sp;
-                        if (stokes<Real>(lut[mid].g, lut[mid].g2, Uniform<Real>::from(r.x), Uniform<Real>::from(r.y),
-                                         cost, sint, phi, cp, sp)) {
+                        phi = (Real)PI_R - phi;
+                        if (phi < (Real)0) phi += TWOPI;
+                    }
+                } else if (cy) {
+                    iy -= sgy;
+                    fx = axis_pos(nx, fx, hx, tmx, t);
+                    fz = axis_pos(nz, fz, hz, tmz, t);
+                    fy = sgy > 0 ? hy : (Real)0;
+                    ny = -ny;
+                    sgy = -sgy;
+                    tmy = t + tdy;
+                    if constexpr (sizeof(Real) == 4) {
+                        spv = -spv;  // phi -> TWOPI - phi
+                    } else {
+                        phi = TWOPI - phi;
+                    }
+                } else {
+                    iz -= sgz;
+                    fx = axis_pos(nx, fx, hx, tmx, t);
+                    fy = axis_pos(ny, fy, hy, tmy, t);
+                    fz = sgz > 0 ? hz : (Real)0;
+                    nz = -nz;
+                    sgz = -sgz;
+                    tmz = t + tdz;
+                }
+            };
+            // Russian roulette of a packet below the threshold; false: it dies
+            auto roulette = [&](uint32_t draw) {
+                const bool live_on = Uniform<Real>::from(draw) < inv_rm;
+                atomicAdd(&s_tal[4], live_on ? (double)(w * (rm - (Real)1)) : -(double)w);
+                if (live_on) w *= rm;
+                return live_on;
+            };
+            // the same set-up for every direction
+            auto setup = [&]() {
+                axis_setup(nx, fx, hx, BIG, tdx, tmx, sgx);
+                axis_setup(ny, fy, hy, BIG, tdy, tmy, sgy);
+                axis_setup(nz, fz, hz, BIG, tdz, tmz, sgz);
+            };
+            if (alive && !go) {
+                if constexpr (sizeof(Real) == 4 && MED != MED_RHOKAP) {
+                    const U4 r = philox4x32_10_rk(ev++, plo, phi32, strm, a.rk);
+                    if (face) {
+                        surface(r.x);
+                    } else {
+                        interact();
+                        cScat += 1;
+                        const bool odd = scatter_f32(hgt[mid], Uniform<Real>::from(r.x), Uniform<Real>::from(r.y), hx, hy, hz,
+                                                     t, fx, fy, fz, nx, ny, nz, sint, cpv, spv, tdx, tdy, tdz, tmx, tmy,
+                                                     tmz, sgx, sgy, sgz);
+                        t = (Real)0;
+                        tau = M<Real>::neglog(Uniform<Real>::from(r.w));
+                        if constexpr (DIST) tau *= inv_mut;
+                        if (odd || !(w >= w_rare)) {
+                            if (!(w > (Real)0)) {
+                                cScat -= 1;
+                                end();
+                            } else if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
+                                atomicOr(&s_err, (unsigned)DEVERR_NAN);
+                                end();
+                            } else {
+                                setup();
+                                if (a.roulette && w < wmin && !roulette(r.z)) end();
+                            }
+                        }
+                    }
+                } else if (face) {
+                    surface(a.fresnel ? philox4x32_10_rk(ev++, plo, phi32, strm, a.rk).x : 0u);
+                } else {
+                    interact();
+                    bool die = !(w > (Real)0);
+                    if (!die) {
+                        const U4 r = philox4x32_10_rk(ev++, plo, phi32, strm, a.rk);
+                        cScat += 1;
+                        fx = axis_pos(nx, fx, hx, tmx, t);
+                        fy = axis_pos(ny, fy, hy, tmy, t);
+                        fz = axis_pos(nz, fz, hz, tmz, t);
+                        Real cost = nz, cp, sp;
+                        if (stokes<Real>(lut[mid].g, lut[mid].g2, Uniform<Real>::from(r.x), Uniform<Real>::from(r.y), cost,
+                                         sint, phi, cp, sp)) {
                             nx = sint * cp;
                             ny = sint * sp;
                             nz = cost;
                         }
-                    }
-                    if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
-                        atomicOr(&s_err, (unsigned)DEVERR_NAN);
-                        die = true;
-                    } else {
-                        axis_setup(nx, fx, hx, BIG, tdx, tmx, sgx);
-                        axis_setup(ny, fy, hy, BIG, tdy, tmy, sgy);
-                        axis_setup(nz, fz, hz, BIG, tdz, tmz, sgz);
-                        t = (Real)0;
-                        if (a.roulette && w < wmin) {
-                            if (Uniform<Real>::from(r.z) < inv_rm) {
-                                atomicAdd(&s_tal[4], (double)(w * (rm - (Real)1)));
-                                w *= rm;
-                            } else {
-                                atomicAdd(&s_tal[4], -(double)w);
-                                die = true;
-                            }
+                        if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
+                            atomicOr(&s_err, (unsigned)DEVERR_NAN);
+                            die = true;
+                        } else {
+                            setup();
+                            t = (Real)0;
+                            die = a.roulette && w < wmin && !roulette(r.z);
+                            tau = M<Real>::neglog(Uniform<Real>::from(r.w));
                         }
-                        tau = M<Real>::neglog(Uniform<Real>::from(r.w));
-                        if constexpr (DIST) tau *= inv_mut;
                     }
-                    if (!die) mode = M_FLY;
-                }
-                if (die) {
-                    if (dep != (Real)0) deposit<T32>(a, cidx, ix, iy, iz, dep);
-                    dep = (Real)0;
-                    cSteps += nsteps;
-                    mode = M_DEAD;
+                    if (die) end();
                 }
             }
         }
@@ -586,12 +656,11 @@ cudaError_t launch_t(const TransportArgs &a, int sm_count, cudaStream_t s)
     const int scat_min = a.scat_min > 0 ? a.scat_min : 20;
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
-    int64_t blocks = (int64_t)sm_count * per_sm;
-    const int64_t need = (a.n + TPB - 1) / TPB;
-    if (blocks > need) blocks = need;
-    if (blocks < 1) blocks = 1;
+    const int per_warp = packets_per_warp(a.n, (int64_t)sm_count * (TPB / 32));
+    const int64_t per_block = (int64_t)per_warp * (TPB / 32);
+    const int64_t blocks = std::min((int64_t)sm_count * per_sm, (a.n + per_block - 1) / per_block);
     count_launch();
-    transport_kernel<Real, MED, T32><<<(unsigned)blocks, TPB, 0, s>>>(a, scat_min);
+    transport_kernel<Real, MED, T32><<<(unsigned)blocks, TPB, 0, s>>>(a, scat_min, 0xffffffffu >> (32 - per_warp));
     return cudaGetLastError();
 }
 

@@ -15,6 +15,9 @@
 // in that instance's own pass; escape weights and step / scatter counts
 // accumulate per instance in shared memory and go to each instance's tally
 // at the end.
+#include <algorithm>
+#include <type_traits>
+
 #include "tam_device.cuh"
 #include "tam_kernels.h"
 #include "transport_common.cuh"
@@ -27,14 +30,16 @@ constexpr int BTPB = 256;
 
 __global__ void __launch_bounds__(BTPB, 4)
     batch_transport_kernel(const BatchTrInst *__restrict__ insts, int ninst, int64_t total,
-                           unsigned long long *work, int scat_min)
+                           unsigned long long *work, int scat_min, unsigned lanes)
 {
     __shared__ BatchTrInst s_in[MAX_BATCH_TR];
     __shared__ int64_t s_first[MAX_BATCH_TR];
     __shared__ double s_tal[MAX_BATCH_TR][5];  // specular, reflected, transmitted, side, roulette net
     __shared__ unsigned long long s_cnt[MAX_BATCH_TR][2];  // voxel steps, scatters
+    __shared__ HgF s_hg[MAX_BATCH_TR];
     for (int t = threadIdx.x; t < ninst; t += blockDim.x) {
         s_in[t] = insts[t];
+        s_hg[t] = hg_consts(insts[t].g, insts[t].g2);
         s_first[t] = insts[t].first;
         for (int k = 0; k < 5; ++k) s_tal[t][k] = 0.0;
         s_cnt[t][0] = s_cnt[t][1] = 0ull;
@@ -46,12 +51,13 @@ __global__ void __launch_bounds__(BTPB, 4)
     const float TWOPI = (float)TWOPI_R;
     const unsigned lane = threadIdx.x & 31u;
 
-    int mode = M_DEAD;
+    bool alive = false;
     bool exhausted = false;
     int inst = 0;
-    int NX = 1, NY = 1, NZ = 1, SZ = 1;  // the lane's instance: grid
-    float mua = 0.f;                     // ... and absorption
-    int ix = 0, iy = 0, iz = 0, cidx = 0, sgx = 1, sgy = 1, sgz = 1, fax = 0;
+    int NX = 1, NY = 1, NZ = 1;  // the lane's instance: grid
+    float mua = 0.f;             // ... and absorption
+    int ix = 0, iy = 0, iz = 0, sgx = 1, sgy = 1, sgz = 1;
+    auto cell = [&]() { return ix + NX * (iy + NY * iz); };
     float fx = 0, fy = 0, fz = 0, nx = 0, ny = 0, nz = 0, sint = 0;
     float cpv = 1, spv = 0;
     float tdx = 0, tdy = 0, tdz = 0, tmx = 0, tmy = 0, tmz = 0, t = 0;
@@ -65,19 +71,20 @@ __global__ void __launch_bounds__(BTPB, 4)
     auto retire = [&]() {
         atomicAdd(&s_cnt[inst][0], (unsigned long long)(uint32_t)(s_in[inst].max_steps - left));
         atomicAdd(&s_cnt[inst][1], (unsigned long long)nscat);
-        mode = M_DEAD;
+        alive = false;
     };
 
     for (;;) {
         // ---------------------------------------------- refill dead lanes --
-        const unsigned need = exhausted ? 0u : __ballot_sync(FULL, mode == M_DEAD);
-        if (need && (__popc(need) >= TAM_REFILL_MIN || need == FULL)) {
+        unsigned live = __ballot_sync(FULL, alive);
+        const unsigned need = exhausted ? 0u : ~live & lanes;
+        if (need && (__popc(need) >= TAM_REFILL_MIN || live == 0u)) {
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if ((int)lane == leader) base = atomicAdd(work, (unsigned long long)__popc(need));
             base = __shfl_sync(FULL, base, leader);
             exhausted = base + (unsigned long long)__popc(need) >= (unsigned long long)total;
-            if (mode == M_DEAD) {
+            if (need >> lane & 1u) {
                 const unsigned long long my = base + __popc(need & ((1u << lane) - 1u));
                 if (my < (unsigned long long)total) {
                     // the packet's instance: the last whose first packet is <= my
@@ -92,7 +99,6 @@ __global__ void __launch_bounds__(BTPB, 4)
                     NX = I.nx;
                     NY = I.ny;
                     NZ = I.nz;
-                    SZ = I.nx * I.ny;
                     mua = I.mua;
                     // launch (src/sourceph.f90:7-49 with the Gaussian beam)
                     const uint64_t pid = (uint64_t)((int64_t)my - I.first);
@@ -124,7 +130,6 @@ __global__ void __launch_bounds__(BTPB, 4)
                         ix = ix > NX - 1 ? NX - 1 : ix;
                         iy = iy > NY - 1 ? NY - 1 : iy;
                         iz = NZ - 1;
-                        cidx = ix + NX * iy + SZ * iz;
                         fx = X - (float)ix * I.hx;
                         fy = Y - (float)iy * I.hy;
                         fz = I.hz - 1.e-8f * I.hz;
@@ -145,153 +150,169 @@ __global__ void __launch_bounds__(BTPB, 4)
                         axis_setup(nz, fz, I.hz, BIG, tdz, tmz, sgz);
                         t = 0.f;
                         dep = 0.f;
-                        mode = M_FLY;
+                        alive = true;
                     }
                 }
             }
+            live = __ballot_sync(FULL, alive);
         }
-        // ------------------------------------------------- flight phase --
-        unsigned sc, fl;
-        auto vstep = [&]() {
-            if (mode != M_FLY) return;
-            if (left-- == 0u) {
-                // past the cap (left wraps: cap - left = cap + 1 steps, as the single pass counts)
-                if (dep != 0.f) atomicAdd(jm + cidx, (double)dep);
-                dep = 0.f;
-                atomicAdd(s_in[inst].tally + T_OVERFLOW, 1.0);
-                atomicOr(s_in[inst].err, (unsigned)DEVERR_STEP_CAP);
-                retire();
-                return;
-            }
-            // nearest face; ties go z over y over x (src/inttau2.f90:116-118)
-            int ax = 2;
-            float tmin = tmz;
-            if (tmy < tmin) { tmin = tmy; ax = 1; }
-            if (tmx < tmin) { tmin = tmx; ax = 0; }
-            const bool cross = tmin < tau;
-            const float tend = cross ? tmin : tau;
-            float dw = tend - t;
-            dw = dw < 0.f ? 0.f : dw;
-            dep += w * dw * mua;
-            t = tend;
-            if (!cross) {
-                mode = M_SCAT;  // the interaction point lies in this cell
-                return;
-            }
-            const bool cx = ax == 0, cy = ax == 1, cz = ax == 2;
-            const int sg = cx ? sgx : (cy ? sgy : sgz);
-            const int j = (cx ? ix : (cy ? iy : iz)) + sg;
-            const int N = cx ? NX : (cy ? NY : NZ);
-            atomicAdd(jm + cidx, (double)dep);
-            dep = 0.f;
-            if ((unsigned)j < (unsigned)N) {
-                ix = cx ? j : ix;
-                iy = cy ? j : iy;
-                iz = cz ? j : iz;
-                cidx += cx ? sg : (cy ? sg * NX : sg * SZ);
-                tmx = cx ? tmx + tdx : tmx;
-                tmy = cy ? tmy + tdy : tmy;
-                tmz = cz ? tmz + tdz : tmz;
-            } else if (s_in[inst].fresnel) {
-                fax = ax;
-                mode = M_FACE;  // on an outer face: the Fresnel draw waits for the event batch
-            } else {
-                atomicAdd(&s_tal[inst][cz ? (sgz > 0 ? 1 : 2) : 3], (double)w);
-                retire();
-            }
-        };
-        for (;;) {
-#pragma unroll
-            for (int q = 0; q < TAM_VSTEPS; ++q) vstep();
-            sc = __ballot_sync(FULL, mode >= M_SCAT);
-            fl = __ballot_sync(FULL, mode == M_FLY);
-            if (fl == 0 || __popc(sc) >= scat_min || (!exhausted && __popc(~(sc | fl)) >= TAM_REFILL_MIN)) break;
-        }
-        if ((sc | fl) == 0) {
+        if (live == 0u) {
             if (exhausted) break;
             continue;
         }
+        // ------------------------------------------------- flight phase --
+        // the single pass's straight-line step (transport.cu): `go` lanes
+        // cross their next face, the others wait for the event batch
+        float tmin;
+        bool py, pz;
+        auto look = [&]() {
+            // nearest face; ties go z over y over x (src/inttau2.f90:116-118)
+            tmin = fminf(fminf(tmx, tmy), tmz);
+            pz = tmz == tmin;
+            py = tmy == tmin && !pz;
+            return tmin < tau;
+        };
+        bool go = look() && alive, capped = false;
+        auto vstep = [&](auto careful) {
+            if constexpr (decltype(careful)::value) {
+                // past the cap (left wraps: cap - left = cap + 1 steps, as the single pass counts)
+                if (go && left == 0u) {
+                    left -= 1u;
+                    capped = true;
+                    go = false;
+                }
+            }
+            left -= go ? 1u : 0u;
+            const float d = dep + w * (tmin - t) * mua;
+            if (go) atomicAdd(jm + cell(), (double)d);
+            dep = go ? 0.f : dep;
+            t = go ? tmin : t;
+            const bool cz = go && pz, cy = go && py, cx = go && !pz && !py;
+            tmx = cx ? tmx + tdx : tmx;
+            tmy = cy ? tmy + tdy : tmy;
+            tmz = cz ? tmz + tdz : tmz;
+            ix += cx ? sgx : 0;
+            iy += cy ? sgy : 0;
+            iz += cz ? sgz : 0;
+            // past an outer face the lane waits for the event batch
+            go = go && (unsigned)ix < (unsigned)NX && (unsigned)iy < (unsigned)NY && (unsigned)iz < (unsigned)NZ;
+            go = look() && go;
+        };
+        {
+            const int thr = wait_min(scat_min, __popc(live));
+            // a flight crosses at most NX + NY + NZ faces between two outer faces
+            if (!__any_sync(FULL, alive && left < (uint32_t)(NX + NY + NZ + 2))) {
+                for (;;) {
+                    const unsigned fl = __ballot_sync(FULL, go);
+                    if (fl == 0u || __popc(live & ~fl) >= thr) break;
+                    int g = go;
+                    uint32_t n = 0;
+                    fly_steps(tmx, tmy, tmz, t, dep, tmin, ix, iy, iz, n, g, tdx, tdy, tdz, w, mua, tau, sgx, sgy, sgz, NX,
+                              NY, NZ, jm);
+                    go = g != 0;
+                    left -= n;
+                }
+            } else {
+                for (;;) {
+                    const unsigned fl = __ballot_sync(FULL, go);
+                    if (fl == 0u || __popc(live & ~fl) >= thr) break;
+                    vstep(std::true_type{});
+                }
+                // the interaction counts as a step too
+                const bool in = (unsigned)ix < (unsigned)NX && (unsigned)iy < (unsigned)NY && (unsigned)iz < (unsigned)NZ;
+                if (alive && !go && !capped && in && left == 0u) {
+                    left -= 1u;
+                    capped = true;
+                }
+                if (capped) {
+                    if (dep != 0.f) atomicAdd(jm + cell(), (double)dep);
+                    dep = 0.f;
+                    atomicAdd(s_in[inst].tally + T_OVERFLOW, 1.0);
+                    atomicOr(s_in[inst].err, (unsigned)DEVERR_STEP_CAP);
+                    retire();
+                }
+            }
+        }
 
         // ------------------------------------------------- event batch --
-        if (sc && (__popc(sc) >= scat_min || fl == 0)) {
-            if (mode >= M_SCAT) {
+        {
+            if (alive && !go) {
                 const BatchTrInst &I = s_in[inst];
-                const bool face = mode == M_FACE;
-                if (!face) w *= I.alb;
-                bool die = !face && !(w > 0.f);
-                U4 r{0u, 0u, 0u, 0u};
-                if (!die) r = philox4x32_10(ev++, plo, phi32, I.stream, (uint32_t)I.seed, (uint32_t)(I.seed >> 32));
-                if (face) {
-                    const bool cx = fax == 0, cy = fax == 1;
-                    const float nc = cx ? nx : (cy ? ny : nz);
-                    if (Uniform<float>::from(r.x) < fresnel<float>(I.n, I.namb, M<float>::abs(nc))) {
-                        // reflect: mirror the crossed component; the next face along it is a cell width back
-                        if (cx) {
-                            fy = axis_pos(ny, fy, I.hy, tmy, t);
-                            fz = axis_pos(nz, fz, I.hz, tmz, t);
-                            fx = sgx > 0 ? I.hx : 0.f;
-                            nx = -nx;
-                            sgx = -sgx;
-                            tmx = t + tdx;
-                            cpv = -cpv;
-                        } else if (cy) {
-                            fx = axis_pos(nx, fx, I.hx, tmx, t);
-                            fz = axis_pos(nz, fz, I.hz, tmz, t);
-                            fy = sgy > 0 ? I.hy : 0.f;
-                            ny = -ny;
-                            sgy = -sgy;
-                            tmy = t + tdy;
-                            spv = -spv;
-                        } else {
-                            fx = axis_pos(nx, fx, I.hx, tmx, t);
-                            fy = axis_pos(ny, fy, I.hy, tmy, t);
-                            fz = sgz > 0 ? I.hz : 0.f;
-                            nz = -nz;
-                            sgz = -sgz;
-                            tmz = t + tdz;
-                        }
-                        mode = M_FLY;
-                    } else {
-                        atomicAdd(&s_tal[inst][(!cx && !cy) ? (sgz > 0 ? 1 : 2) : 3], (double)w);
-                        retire();
-                    }
-                } else if (!die) {
-                    nscat += 1;
-                    fx = axis_pos(nx, fx, I.hx, tmx, t);
-                    fy = axis_pos(ny, fy, I.hy, tmy, t);
-                    fz = axis_pos(nz, fz, I.hz, tmz, t);
-                    float cost = nz;
-                    if (stokes_f32(I.g, I.g2, Uniform<float>::from(r.x), Uniform<float>::from(r.y), cost, sint, cpv,
-                                   spv)) {
-                        nx = sint * cpv;
-                        ny = sint * spv;
-                        nz = cost;
-                    }
-                    if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
-                        atomicOr(I.err, (unsigned)DEVERR_NAN);
-                        die = true;
-                    } else {
-                        axis_setup(nx, fx, I.hx, BIG, tdx, tmx, sgx);
-                        axis_setup(ny, fy, I.hy, BIG, tdy, tmy, sgy);
-                        axis_setup(nz, fz, I.hz, BIG, tdz, tmz, sgz);
-                        t = 0.f;
-                        if (I.roulette && w < I.wmin) {
-                            if (Uniform<float>::from(r.z) < I.inv_rm) {
-                                atomicAdd(&s_tal[inst][4], (double)(w * (I.rm - 1.f)));
-                                w *= I.rm;
-                            } else {
-                                atomicAdd(&s_tal[inst][4], -(double)w);
-                                die = true;
-                            }
-                        }
-                        tau = M<float>::neglog(Uniform<float>::from(r.w)) * I.inv_mut;
-                    }
-                    if (!die) mode = M_FLY;
-                }
-                if (die) {
-                    if (dep != 0.f) atomicAdd(jm + cidx, (double)dep);
+                const bool cx = (unsigned)ix >= (unsigned)NX, cy = (unsigned)iy >= (unsigned)NY;
+                const bool cz = (unsigned)iz >= (unsigned)NZ;
+                // the packet's end inside the grid
+                auto end = [&]() {
+                    if (dep != 0.f) atomicAdd(jm + cell(), (double)dep);
                     dep = 0.f;
                     retire();
+                };
+                const U4 r = philox4x32_10(ev++, plo, phi32, I.stream, (uint32_t)I.seed, (uint32_t)(I.seed >> 32));
+                if (cx || cy || cz) {
+                    const float nc = cx ? nx : (cy ? ny : nz);
+                    if (!I.fresnel || !(Uniform<float>::from(r.x) < fresnel<float>(I.n, I.namb, M<float>::abs(nc)))) {
+                        // escape (nothing to deposit: the crossing did)
+                        atomicAdd(&s_tal[inst][cz ? (sgz > 0 ? 1 : 2) : 3], (double)w);
+                        retire();
+                    } else if (cx) {
+                        // reflect, back into the cell it came from: mirror the crossed component; the next face along
+                        // it is a cell width back
+                        ix -= sgx;
+                        fy = axis_pos(ny, fy, I.hy, tmy, t);
+                        fz = axis_pos(nz, fz, I.hz, tmz, t);
+                        fx = sgx > 0 ? I.hx : 0.f;
+                        nx = -nx;
+                        sgx = -sgx;
+                        tmx = t + tdx;
+                        cpv = -cpv;
+                    } else if (cy) {
+                        iy -= sgy;
+                        fx = axis_pos(nx, fx, I.hx, tmx, t);
+                        fz = axis_pos(nz, fz, I.hz, tmz, t);
+                        fy = sgy > 0 ? I.hy : 0.f;
+                        ny = -ny;
+                        sgy = -sgy;
+                        tmy = t + tdy;
+                        spv = -spv;
+                    } else {
+                        iz -= sgz;
+                        fx = axis_pos(nx, fx, I.hx, tmx, t);
+                        fy = axis_pos(ny, fy, I.hy, tmy, t);
+                        fz = sgz > 0 ? I.hz : 0.f;
+                        nz = -nz;
+                        sgz = -sgz;
+                        tmz = t + tdz;
+                    }
+                } else {
+                    // on to the interaction point inside this cell (tau: its distance along the flight)
+                    left -= 1u;
+                    dep += w * (tau - t) * mua;
+                    t = tau;
+                    w *= I.alb;
+                    nscat += 1;
+                    const bool odd = scatter_f32(s_hg[inst], Uniform<float>::from(r.x), Uniform<float>::from(r.y), I.hx, I.hy,
+                                                 I.hz, t, fx, fy, fz, nx, ny, nz, sint, cpv, spv, tdx, tdy, tdz, tmx, tmy,
+                                                 tmz, sgx, sgy, sgz);
+                    t = 0.f;
+                    tau = M<float>::neglog(Uniform<float>::from(r.w)) * I.inv_mut;
+                    if (odd || !(w > 0.f) || (I.roulette && w < I.wmin)) {
+                        if (!(w > 0.f)) {
+                            nscat -= 1;
+                            end();
+                        } else if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
+                            atomicOr(I.err, (unsigned)DEVERR_NAN);
+                            end();
+                        } else {
+                            axis_setup(nx, fx, I.hx, BIG, tdx, tmx, sgx);
+                            axis_setup(ny, fy, I.hy, BIG, tdy, tmy, sgy);
+                            axis_setup(nz, fz, I.hz, BIG, tdz, tmz, sgz);
+                            if (I.roulette && w < I.wmin) {
+                                const bool live_on = Uniform<float>::from(r.z) < I.inv_rm;
+                                atomicAdd(&s_tal[inst][4], live_on ? (double)(w * (I.rm - 1.f)) : -(double)w);
+                                if (live_on) w *= I.rm;
+                                else end();
+                            }
+                        }
+                    }
                 }
             }
         }
@@ -323,12 +344,12 @@ cudaError_t launch_batch_transport(const BatchTrInst *insts, int n, int64_t tota
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_transport_kernel, BTPB, 0);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
-    int64_t blocks = (int64_t)sm_count * per_sm;
-    const int64_t need = (total + BTPB - 1) / BTPB;
-    if (blocks > need) blocks = need;
-    if (blocks < 1) blocks = 1;
+    const int per_warp = packets_per_warp(total, (int64_t)sm_count * (BTPB / 32));
+    const int64_t per_block = (int64_t)per_warp * (BTPB / 32);
+    const int64_t blocks = std::min((int64_t)sm_count * per_sm, (total + per_block - 1) / per_block);
     count_launch();
-    batch_transport_kernel<<<(unsigned)blocks, BTPB, 0, s>>>(insts, n, total, work, scat_min > 0 ? scat_min : 20);
+    batch_transport_kernel<<<(unsigned)blocks, BTPB, 0, s>>>(insts, n, total, work, scat_min > 0 ? scat_min : 20,
+                                                              0xffffffffu >> (32 - per_warp));
     return cudaGetLastError();
 }
 

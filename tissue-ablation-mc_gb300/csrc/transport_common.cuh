@@ -91,6 +91,16 @@ __device__ __forceinline__ float rsqrt_ax(float x)
     return r;
 }
 
+// FP32 constants of one material's HG sampling: with u uniform,
+// t = n1 / (d0 + d1 u) and the cosine is (b0 - t^2) ib.
+struct HgF {
+    float g, n1, d0, d1, b0, ib;
+};
+__device__ __forceinline__ HgF hg_consts(float g, float g2)
+{
+    return HgF{g, 1.f - g2, 1.f - g, 2.f * g, 1.f + g2, rcp_ax(2.f * g)};
+}
+
 // FP32 form of the same HG deflection.  The azimuth is carried as the pair
 // (cos phi, sin phi) and rotated by the deflection angle dph, since
 // phi' = phi +- dph (src/stokes.f90:136-140) gives
@@ -99,11 +109,11 @@ __device__ __forceinline__ float rsqrt_ax(float x)
 // pair is renormalised so that rounding cannot drift over many scatters.
 // Every sampled quantity (t, bmu, ang, cost, cosdph) follows the reference's
 // formulas; only the evaluation of phi differs.
-__device__ __forceinline__ bool stokes_f32(float hgg, float g2, float u0, float u1, float &cost, float &sint, float &cp,
+__device__ __forceinline__ bool stokes_f32(const HgF &c, float u0, float u1, float &cost, float &sint, float &cp,
                                            float &sp)
 {
     const float PI = (float)PI_R, TWOPI = (float)TWOPI_R;
-    if (hgg == 0.f) {
+    if (c.g == 0.f) {
         cost = 2.f * u0 - 1.f;
         const float s2 = 1.f - cost * cost;
         sint = s2 <= 0.f ? 0.f : sqrt_ax(s2);
@@ -111,8 +121,8 @@ __device__ __forceinline__ bool stokes_f32(float hgg, float g2, float u0, float 
         return true;
     }
     const float costp = cost, sintp = sint;
-    const float t = __fdividef(1.f - g2, 1.f - hgg + 2.f * hgg * u0);
-    const float bmu = __fdividef((1.f + g2) - t * t, 2.f * hgg);
+    const float t = c.n1 * rcp_ax(__fmaf_rn(c.d1, u0, c.d0));
+    const float bmu = __fmaf_rn(-t, t, c.b0) * c.ib;
     if (fabsf(bmu) >= 1.f) return false;  // clamped to +-1: direction unchanged
     const float sinbt = sqrt_ax(1.f - bmu * bmu);
     const float ri1 = TWOPI * u1;
@@ -163,11 +173,8 @@ template <typename Real> __device__ __forceinline__ Real clamp0h(Real f, Real h)
 
 // Voxel steps per warp vote of the flight phase: the votes are a sizeable
 // share of a step, and a lane that stops early only idles for the rest (its
-// packet's walk does not depend on when the event batch runs).  Measured on
-// the 200^3 bench pass: 2 -> 190.5, 4 -> 193.5, 6 -> 189.9 Mphotons/s.
-#ifndef TAM_VSTEPS
-#define TAM_VSTEPS 4
-#endif
+// packet's walk does not depend on when the event batch runs).
+constexpr int VSTEPS = 4;
 
 // Dead lanes of a warp that make it draw new packets: the launch code runs
 // for the dead lanes only, so refilling them together spends fewer of its
@@ -178,7 +185,34 @@ template <typename Real> __device__ __forceinline__ Real clamp0h(Real f, Real h)
 #define TAM_REFILL_MIN 2
 #endif
 
-enum : int { M_DEAD = 0, M_FLY = 1, M_SCAT = 2, M_FACE = 3 };  // M_SCAT, M_FACE: waiting for the event batch
+// Lanes that must wait before a warp with `live` live lanes runs its event
+// batch: scat_min of 32, and the same share of fewer (FP32: in FP64 the event
+// batch keeps the FP64 pipe busy as long for few lanes as for many, and taking
+// it earlier costs 7 % on passes of 1e5 packets).
+__device__ __forceinline__ int wait_min(int scat_min, int live)
+{
+    return live >= 31 ? scat_min : max(1, (scat_min * live) >> 5);
+}
+
+// Packets that a warp holds at a time: with fewer packets than lanes, a pass
+// takes as long as its longest packet's walk, whose events wait for those of
+// the other lanes, so a small pass spreads over the SMs, one block each, before
+// its warps fill up.  100^3 cube, FP32, 1 / 4 / 32 packets a warp: 1.08 / 1.16 /
+// 1.33 ms for 1000 packets, 2.2 / 1.83 / 1.91 ms for 10,000, 7.9 / 4.2 / 2.4 ms
+// for 100,000.
+inline int packets_per_warp(int64_t n, int64_t warps)
+{
+    const int64_t k = (n + warps - 1) / warps;
+    return (int)(k < 1 ? 1 : (k > 32 ? 32 : k));
+}
+
+// a < b for values that are not negative (nor NaN): FP64 on the bit patterns,
+// which order alike, off GB300's narrow FP64 pipe.
+__device__ __forceinline__ bool less_pos(float a, float b) { return a < b; }
+__device__ __forceinline__ bool less_pos(double a, double b)
+{
+    return __double_as_longlong(a) < __double_as_longlong(b);
+}
 
 // Per-flight DDA set-up from the in-cell position f and direction n of one
 // axis: td = cell width along the ray, tm = distance to the next face.
@@ -217,6 +251,156 @@ template <typename Real> __device__ __forceinline__ Real axis_pos(Real n, Real f
 {
     const Real r = n > (Real)0 ? h - (tm - t) * n : (n < (Real)0 ? -(tm - t) * n : f);
     return clamp0h(r, h);
+}
+
+// VSTEPS voxel steps (src/inttau2.f90:37-63) of the FP32 distance-tracked
+// flight in a uniform medium, as predicated PTX: per step the deposit of the
+// cell's path (one red.f64), the crossing of the nearest face (ties go z over
+// y over x, src/inttau2.f90:116-118; a two-output setp gives "this axis" and
+// "a later axis" at once) and the test whether the flight goes on (the cell
+// is inside the grid and the next face lies before the interaction point at
+// distance tau).  `go` (0 or 1) and tmin = min(tmx, tmy, tmz) are kept ahead
+// by one step; a lane without `go` is left unchanged.
+//
+// The transport is bound by instruction issue.  As C++ the compiler turns
+// each conditional update into an operation and a select; predicated, a step
+// is 27 instructions against 44.
+#define TAM_VSTEP_PTX                                                                                       \
+    "sub.f32 a, %5, %3;\n\t"                                                                                \
+    "mul.f32 a, %14, a;\n\t"                                                                               \
+    "fma.rn.f32 a, a, %15, %4;\n\t"                                                                        \
+    "mad.lo.s32 c, %8, %21, %7;\n\t"                                                                       \
+    "mad.lo.s32 c, c, %20, %6;\n\t"                                                                        \
+    "mul.wide.s32 l, c, 8;\n\t"                                                                            \
+    "add.s64 l, l, %23;\n\t"                                                                               \
+    "cvt.f64.f32 d, a;\n\t"                                                                             \
+    "@p red.global.add.f64 [l], d;\n\t"                                                                    \
+    "@p mov.f32 %4, 0f00000000;\n\t"                                                                       \
+    "@p mov.f32 %3, %5;\n\t"                                                                               \
+    "@p add.u32 %9, %9, 1;\n\t"                                                                            \
+    "setp.eq.and.f32 pz|q, %2, %5, p;\n\t"                                                                 \
+    "setp.eq.and.f32 py|px, %1, %5, q;\n\t"                                                                \
+    "@px add.f32 %0, %0, %11;\n\t"                                                                         \
+    "@py add.f32 %1, %1, %12;\n\t"                                                                         \
+    "@pz add.f32 %2, %2, %13;\n\t"                                                                         \
+    "@px add.s32 %6, %6, %17;\n\t"                                                                         \
+    "@py add.s32 %7, %7, %18;\n\t"                                                                         \
+    "@pz add.s32 %8, %8, %19;\n\t"                                                                         \
+    "setp.lt.and.u32 p, %6, %20, p;\n\t"                                                                   \
+    "setp.lt.and.u32 p, %7, %21, p;\n\t"                                                                   \
+    "setp.lt.and.u32 p, %8, %22, p;\n\t"                                                                   \
+    "min.f32 %5, %0, %1, %2;\n\t"                                                                          \
+    "setp.lt.and.f32 p, %5, %16, p;\n\t"
+__device__ __forceinline__ void fly_steps(float &tmx, float &tmy, float &tmz, float &t, float &dep, float &tmin, int &ix,
+                                          int &iy, int &iz, uint32_t &nsteps, int &go, float tdx, float tdy, float tdz,
+                                          float w, float mua, float tau, int sgx, int sgy, int sgz, int NX, int NY, int NZ,
+                                          double *tally)
+{
+    static_assert(VSTEPS == 4, "the steps below");
+    asm volatile("{\n\t"
+                 ".reg .pred p, q, px, py, pz;\n\t"
+                 ".reg .f32 a;\n\t"
+                 ".reg .s32 c;\n\t"
+                 ".reg .s64 l;\n\t"
+                 ".reg .f64 d;\n\t"
+                 "setp.ne.s32 p, %10, 0;\n\t"
+                 TAM_VSTEP_PTX TAM_VSTEP_PTX TAM_VSTEP_PTX TAM_VSTEP_PTX
+                 "selp.s32 %10, 1, 0, p;\n\t"
+                 "}"
+                 : "+f"(tmx), "+f"(tmy), "+f"(tmz), "+f"(t), "+f"(dep), "+f"(tmin), "+r"(ix), "+r"(iy), "+r"(iz),
+                   "+r"(nsteps), "+r"(go)
+                 : "f"(tdx), "f"(tdy), "f"(tdz), "f"(w), "f"(mua), "f"(tau), "r"(sgx), "r"(sgy), "r"(sgz), "r"(NX),
+                   "r"(NY), "r"(NZ), "l"(tally)
+                 : "memory");
+}
+#undef TAM_VSTEP_PTX
+
+// The crossing of one step in FP32 without the deposit, for media whose cells
+// differ: the caller deposits before it and looks the new cell up after it.
+// dtx, dty, dtz: what a crossing adds to the crossed axis's face distance;
+// ahead: the optical depth to the face.
+__device__ __forceinline__ void fly_cross(float &tmx, float &tmy, float &tmz, float &t, float &dep, float &tmin, float &tau,
+                                          int &ix, int &iy, int &iz, uint32_t &nsteps, int &go, float dtx, float dty,
+                                          float dtz, float ahead, int sgx, int sgy, int sgz, int NX, int NY, int NZ)
+{
+    asm("{\n\t"
+        ".reg .pred p, q, px, py, pz;\n\t"
+        "setp.ne.s32 p, %11, 0;\n\t"
+        "@p sub.f32 %6, %6, %15;\n\t"
+        "@p mov.f32 %4, 0f00000000;\n\t"
+        "@p mov.f32 %3, %5;\n\t"
+        "@p add.u32 %10, %10, 1;\n\t"
+        "setp.eq.and.f32 pz|q, %2, %5, p;\n\t"
+        "setp.eq.and.f32 py|px, %1, %5, q;\n\t"
+        "@px add.f32 %0, %0, %12;\n\t"
+        "@py add.f32 %1, %1, %13;\n\t"
+        "@pz add.f32 %2, %2, %14;\n\t"
+        "@px add.s32 %7, %7, %16;\n\t"
+        "@py add.s32 %8, %8, %17;\n\t"
+        "@pz add.s32 %9, %9, %18;\n\t"
+        "setp.lt.and.u32 p, %7, %19, p;\n\t"
+        "setp.lt.and.u32 p, %8, %20, p;\n\t"
+        "setp.lt.and.u32 p, %9, %21, p;\n\t"
+        "min.f32 %5, %0, %1, %2;\n\t"
+        "selp.s32 %11, 1, 0, p;\n\t"
+        "}"
+        : "+f"(tmx), "+f"(tmy), "+f"(tmz), "+f"(t), "+f"(dep), "+f"(tmin), "+f"(tau), "+r"(ix), "+r"(iy), "+r"(iz),
+          "+r"(nsteps), "+r"(go)
+        : "f"(dtx), "f"(dty), "f"(dtz), "f"(ahead), "r"(sgx), "r"(sgy), "r"(sgz), "r"(NX), "r"(NY), "r"(NZ));
+}
+
+// Whether a direction lies (nearly) in a plane of the grid: the two functions
+// below do not take it.
+__device__ __forceinline__ bool in_plane(float nx, float ny, float nz)
+{
+    return fminf(fminf(fabsf(nx), fabsf(ny)), fabsf(nz)) < 1e-30f;
+}
+// axis_setup and axis_pos of a component that is not parallel to the faces,
+// and of 0 <= f <= h: the same values (a sign moves through a product, and
+// h - f and f are not negative) with about half the instructions.
+__device__ __forceinline__ void axis_setup_steep(float n, float f, float h, float &td, float &tm, int &sg)
+{
+    const float inv = fabsf(rcp_ax(n));
+    td = h * inv;
+    tm = (n > 0.f ? h - f : f) * inv;
+    sg = n > 0.f ? 1 : -1;
+}
+__device__ __forceinline__ float axis_pos_steep(float n, float h, float tm, float t)
+{
+    const float e = tm - t;
+    const float r = n > 0.f ? __fmaf_rn(-e, n, h) : -e * n;
+    return fminf(fmaxf(r, 0.f), h);
+}
+
+// One FP32 scatter: the packet's in-cell position at distance t of its
+// flight, the HG rotation of its direction, and the new flight's set-up.
+// True when the new direction needs a closer look (NaN, or in a plane of the
+// grid: the face distances then come from axis_setup); the test, a few
+// instructions and rarely true, stands in for a branch at each of its parts.
+__device__ __forceinline__ bool scatter_f32(const HgF &hg, float u0, float u1, float hx, float hy, float hz, float t,
+                                            float &fx, float &fy, float &fz, float &nx, float &ny, float &nz, float &sint,
+                                            float &cpv, float &spv, float &tdx, float &tdy, float &tdz, float &tmx,
+                                            float &tmy, float &tmz, int &sgx, int &sgy, int &sgz)
+{
+    if (in_plane(nx, ny, nz)) {
+        fx = axis_pos(nx, fx, hx, tmx, t);
+        fy = axis_pos(ny, fy, hy, tmy, t);
+        fz = axis_pos(nz, fz, hz, tmz, t);
+    } else {
+        fx = axis_pos_steep(nx, hx, tmx, t);
+        fy = axis_pos_steep(ny, hy, tmy, t);
+        fz = axis_pos_steep(nz, hz, tmz, t);
+    }
+    float cost = nz;
+    if (stokes_f32(hg, u0, u1, cost, sint, cpv, spv)) {
+        nx = sint * cpv;
+        ny = sint * spv;
+        nz = cost;
+    }
+    axis_setup_steep(nx, fx, hx, tdx, tmx, sgx);
+    axis_setup_steep(ny, fy, hy, tdy, tmy, sgy);
+    axis_setup_steep(nz, fz, hz, tdz, tmz, sgz);
+    return in_plane(nx, ny, nz) || !(nz == nz) || !(nx == nx) || !(ny == ny);
 }
 
 }  // namespace
