@@ -153,6 +153,11 @@ struct tam_ctx {
     bool use_slab = true;            // class-table step: the slab form where the grid allows it
     uint8_t *d_cls = nullptr;
     int cls_pitch = 0;
+    // FP64 contexts: the class tables and grid of the class-table step; the
+    // grid is made from k, rho, c when a heat call first needs it
+    tam::ClassLut64 clut64{};
+    uint8_t *d_cls64 = nullptr;
+    bool cls64_ok = false;
     bool thermal_by_class = false;
     int cls_uniform = -1;            // >= 0 while every voxel has this thermal class
     tam::ClassLut clut{};
@@ -429,16 +434,23 @@ int set_thermal_classes(tam_ctx *ctx, int u)
         L.rho[i] = (float)ri;
         L.c[i] = (float)ci;
         L.irc[i] = (float)(1.0 / (ri * ci));
+        tam::ClassLut64 &D = ctx->clut64;
+        D.k[i] = ki;
+        D.rho[i] = ri;
+        D.c[i] = ci;
+        D.irc[i] = 1.0 / (ri * ci);
         for (int j = 0; j < tam::MAX_MAT; ++j) {
             const int b = j < nm ? j : 0;
             const double kf = 0.5 * (ki + ctx->lut.k[b]), rf = 0.5 * (ri + ctx->lut.rho[b]),
                          cf = 0.5 * (ci + ctx->lut.c[b]);
-            L.fa[i * tam::MAX_MAT + j] = (float)(kf / (rf * cf));
+            D.fa[i * tam::MAX_MAT + j] = kf / (rf * cf);
+            L.fa[i * tam::MAX_MAT + j] = (float)D.fa[i * tam::MAX_MAT + j];
         }
     }
     ctx->cls_uniform = u;
-    L.uniform = u;
+    L.uniform = ctx->clut64.uniform = u;
     ctx->thermal_by_class = true;
+    ctx->cls64_ok = false;
     if (ctx->d_cls)
         CK(tam::launch_cls_from_mat(ctx->d_mat, nm, ctx->d_cls, ctx->nx, ctx->ny, ctx->nz, ctx->cls_pitch, ctx->stream));
     if (ctx->d_cls && ctx->fslab && u < 0) CK(tam::fused_slab_tile_flags(ctx->fslab, ctx->zchunk, ctx->stream));
@@ -924,8 +936,25 @@ int slab_lists(tam_ctx *ctx)
     return TAM_OK;
 }
 
+// The class grid of an FP64 context's class-table step.  Without the memory for
+// it the per-voxel step runs.
+int cls64_setup(tam_ctx *ctx)
+{
+    if (!ctx->fp64 || !ctx->use_cls || !ctx->thermal_by_class || ctx->cls_uniform >= 0 || ctx->cls64_ok) return TAM_OK;
+    if (!ctx->d_cls64 && dalloc_t(ctx, &ctx->d_cls64, ctx->ni) != TAM_OK) {
+        ctx->d_cls64 = nullptr;
+        ctx->err.clear();
+        return TAM_OK;
+    }
+    CK(tam::launch_cls_from_props((const double *)ctx->d_k, (const double *)ctx->d_rho, (const double *)ctx->d_c,
+                                  ctx->clut64, std::min(ctx->cfg.nmat, (int)tam::MAX_MAT), ctx->d_cls64, ctx->ni,
+                                  ctx->stream));
+    ctx->cls64_ok = true;
+    return TAM_OK;
+}
+
 // Forms of the config-mode heat step, by what the context's state allows.
-enum HeatForm { HF_CLS = 0, HF_STAGED, HF_TMA, HF_CPASYNC, HF_SLAB };
+enum HeatForm { HF_CLS = 0, HF_STAGED, HF_TMA, HF_CPASYNC, HF_SLAB, HF_CLS64 };
 
 HeatForm heat_form(const tam_ctx *ctx)
 {
@@ -933,6 +962,7 @@ HeatForm heat_form(const tam_ctx *ctx)
     if (ctx->fcls && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class) return HF_CLS;
     if (!ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && ctx->d_cls) return HF_STAGED;
     if (ctx->tma && ctx->use_tma) return HF_TMA;
+    if (ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && (ctx->cls_uniform >= 0 || ctx->cls64_ok)) return HF_CLS64;
     return HF_CPASYNC;
 }
 
@@ -955,6 +985,7 @@ int launch_heat(tam_ctx *ctx, tam::FusedArgs &a, HeatForm form, int which, cudaS
         break;
     }
     case HF_TMA: CK(tam::launch_fused_tma(a, ctx->tma, which, s)); break;
+    case HF_CLS64: CK(tam::launch_cls64_step(a, ctx->clut64, ctx->d_cls64, s)); break;
     default: CK(tam::launch_fused_step(a, ctx->fp64, s)); break;
     }
     // tissue left with six air neighbours turns to air (src/3dFD.f90:347-349)
@@ -1041,6 +1072,7 @@ int cfg_heat(tam_ctx *ctx, int32_t nsteps, int32_t *done = nullptr, bool stop_on
 {
     tam::FusedArgs a = fused_args(ctx);
     const int check = ctx->cfg.retrace_check > 0 ? ctx->cfg.retrace_check : (stop_on_trace ? 1 : 0);
+    if (nsteps > 0) RC(cls64_setup(ctx));
     const HeatForm form = heat_form(ctx);
     if (form == HF_STAGED && nsteps > 0) RC(staged_setup(ctx));
     if (form == HF_TMA && ctx->coeff_dirty && nsteps > 0) {
@@ -2976,7 +3008,8 @@ void set_scalars(tam_ctx *c, const Scalars &S)
     c->cls_uniform = S.cls_uniform;
     c->thermal_by_class = S.thermal_by_class != 0;
     c->since_check = S.since_check;
-    c->clut.uniform = S.cls_uniform;
+    c->clut.uniform = c->clut64.uniform = S.cls_uniform;
+    c->cls64_ok = false;
     c->mc_passes = S.mc_passes;
     c->nabl_at_trace = S.nabl_at_trace;
     c->nabl_at_uniform = S.nabl_at_uniform;
@@ -3042,6 +3075,7 @@ int tam_load_state(tam_ctx *ctx, const char *path)
         return fail(ctx, TAM_E_STATE, "state file was written by a context with other parameters");
     const auto bufs = state_buffers(ctx);
     if (nb != bufs.size()) return fail(ctx, TAM_E_STATE, "state file holds another set of fields");
+    ctx->cls64_ok = false;  // made again from the k, rho, c loaded below
     std::vector<char> host;
     CK(cudaStreamSynchronize(ctx->stream));
     for (const auto &b : bufs) {

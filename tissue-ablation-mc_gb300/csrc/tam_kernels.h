@@ -292,6 +292,19 @@ struct ClassLut {
     float k[MAX_MAT], rho[MAX_MAT], c[MAX_MAT];
     int32_t uniform;              // >= 0: every voxel has this class
 };
+// FP64 step on thermal classes (heat64.cu): the tables in FP64, and the class
+// of every voxel (x fastest, no padding; not read when uniform >= 0).
+struct ClassLut64 {
+    double fa[MAX_MAT * MAX_MAT];
+    double irc[MAX_MAT];
+    double k[MAX_MAT], rho[MAX_MAT], c[MAX_MAT];
+    double hdk[6 * MAX_MAT];      // Robin faces: h d / k per face and class (filled by the launcher)
+    int32_t uniform;
+};
+cudaError_t launch_cls64_step(const FusedArgs &a, const ClassLut64 &L, const uint8_t *cls, cudaStream_t s);
+// The class grid of that step from per-voxel k, rho, c, each those of a class.
+cudaError_t launch_cls_from_props(const double *k, const double *rho, const double *c, const ClassLut64 &L, int ncls,
+                                  uint8_t *cls, int64_t n, cudaStream_t s);
 struct FusedCls;  // opaque: tensor maps of T[2], Tc[2], J and the class grid
 int cls_pitch_for(int nx);
 cudaError_t launch_cls_from_mat(const uint8_t *mat, int nmat, uint8_t *cls, int nx, int ny, int nz, int pitch,

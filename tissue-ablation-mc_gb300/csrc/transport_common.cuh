@@ -5,6 +5,7 @@
 // set-up and position reconstruction.
 #pragma once
 
+#include "ieee_bits.h"
 #include "tam_device.cuh"
 #include "tam_kernels.h"
 
@@ -211,7 +212,7 @@ inline int packets_per_warp(int64_t n, int64_t warps)
 __device__ __forceinline__ bool less_pos(float a, float b) { return a < b; }
 __device__ __forceinline__ bool less_pos(double a, double b)
 {
-    return __double_as_longlong(a) < __double_as_longlong(b);
+    return (int64_t)ieee::bits(a) < (int64_t)ieee::bits(b);
 }
 
 // Per-flight DDA set-up from the in-cell position f and direction n of one
