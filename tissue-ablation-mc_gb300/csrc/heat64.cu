@@ -11,8 +11,9 @@
 // source's 1 / (rho c) per voxel, ~280 FP64 operations.  With classes, those
 // are looked up (face coefficients per class pair, computed on the host with
 // the same means), dt is folded into them, and screens are integer compares
-// of the bit patterns: 14 FP64 operations per voxel in one class, 20 in
-// several.  100^3 cube: 443 -> 45 us per step.
+// of the bit patterns: 13 FP64 operations per voxel in one class, 18 in
+// several.  100^3 cube with a core in the damage window: 443 -> 54 us per step
+// (FP64 pipe 76 % busy; a third of its operations are the window's).
 #include <algorithm>
 
 #include "heat_common.cuh"
@@ -22,26 +23,37 @@ namespace tam {
 
 namespace {
 
-constexpr int CX = 32, CY = 8;  // voxels of a block's column tile
+constexpr int TPB64 = 128;
+constexpr int ROWS = 2;  // y-adjacent voxels of a thread
+constexpr int ZMAX = 16;  // planes per block at most (the list holds every voxel of a block)
 
+// A thread marches ROWS y-adjacent columns through zchunk planes; the threads
+// of a block take consecutive columns of the x-y plane (x fastest, wrapping from
+// row pair to row pair), so every lane works at any nx.  Face differences are
+// formed once where both voxels are the thread's: along z from plane to plane,
+// along y inside the pair.  Voxels in the damage window (whose exponential and
+// quotient are ~50 FP64 operations) or at ablation are listed and taken once the
+// planes are done, a full warp at a time.
 template <bool UNIFORM>
-__global__ void __launch_bounds__(CX *CY) cls64_step_kernel(const __grid_constant__ FusedArgs a,
-                                                            const __grid_constant__ ClassLut64 L, const uint8_t *cls,
-                                                            int zchunk)
+__global__ void __launch_bounds__(TPB64) cls64_step_kernel(const __grid_constant__ FusedArgs a,
+                                                           const __grid_constant__ ClassLut64 L, const uint8_t *cls,
+                                                           int zchunk)
 {
     __shared__ double s_fa[UNIFORM ? 1 : MAX_MAT * MAX_MAT], s_src[UNIFORM ? 1 : MAX_MAT];
-    const int x = blockIdx.x * CX + threadIdx.x, y = blockIdx.y * CY + threadIdx.y;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const double Pdt = step_pdt<double>(a), t_new = step_tnew(a);
     const bool src_on = Pdt != 0.0;
     if (!UNIFORM) {
-        const int tid = threadIdx.y * CX + threadIdx.x;
-        s_fa[tid] = L.fa[tid];
-        if (tid < MAX_MAT) s_src[tid] = Pdt * L.irc[tid];
-        __syncthreads();
+        for (int t = threadIdx.x; t < MAX_MAT * MAX_MAT; t += TPB64) s_fa[t] = L.fa[t];
+        if (threadIdx.x < MAX_MAT) s_src[threadIdx.x] = Pdt * L.irc[threadIdx.x];
     }
-    if (x >= nx || y >= ny) return;
-    const int z0 = blockIdx.z * zchunk, z1 = min(nz, z0 + zchunk);
+    __shared__ unsigned short s_list[TPB64 * ROWS * ZMAX];
+    __shared__ int s_cnt;
+    if (threadIdx.x == 0) s_cnt = 0;
+    __syncthreads();
+    const int64_t col0 = blockIdx.x * (int64_t)TPB64, col = col0 + threadIdx.x;
+    const int x = (int)(col % nx), y0 = (int)(col / nx) * ROWS;
+    const int z0 = blockIdx.y * zchunk, z1 = min(nz, z0 + zchunk);
     const int64_t sy = nx, sz = (int64_t)nx * ny, ni = sz * nz;
     const double *T = (const double *)a.T_in;
     double *To = (double *)a.T_out;
@@ -55,65 +67,100 @@ __global__ void __launch_bounds__(CX *CY) cls64_step_kernel(const __grid_constan
     // negative and NaN ones
     const uint64_t screen = ieee::bits(a.dc[FC_SCREEN]);
     const uint64_t boil = a.boil ? ieee::bits(a.dc[FC_TBOIL]) : ~0ull;
-    int64_t v = x + sy * y + sz * z0;
     auto klass = [&](int64_t q) -> int { return UNIFORM ? uc : (int)__ldg(cls + q); };
-    // neighbour difference across face f: towards the neighbour n, or the ghost's
-    // (Dirichlet: the face's temperature; Robin: -h d / k (T - T_amb))
-    auto face = [&](bool inside, int f, int64_t n, double tc, int k) -> double {
-        double t = a.dc[FC_BCT + f];
-        if (inside) t = __ldg(T + n);
-        else if (a.bc_type[f] == BC_ROBIN) return -L.hdk[f * MAX_MAT + k] * (tc - a.dc[FC_BCTA + f]);
-        return t - tc;
+    // difference towards the neighbour n across face f, or the face's ghost
+    // (Dirichlet: the face's temperature; Robin: -h d / k (T - T_amb)); in a
+    // grid of several classes times the face's diffusivity
+    auto flux = [&](bool inside, int f, int64_t n, double tc, int k) -> double {
+        double d;
+        if (!inside && a.bc_type[f] == BC_ROBIN) d = -L.hdk[f * MAX_MAT + k] * (tc - a.dc[FC_BCTA + f]);
+        else d = (inside ? __ldg(T + n) : a.dc[FC_BCT + f]) - tc;
+        return UNIFORM ? d : s_fa[k * MAX_MAT + (inside ? klass(n) : k)] * d;
     };
-    double tc = T[v], tm = z0 > 0 ? T[v - sz] : 0.0;
-    int kc = klass(v), km = z0 > 0 ? klass(v - sz) : kc;
+    double tc[ROWS], fzm[ROWS];
+    int kc[ROWS];
+    bool in[ROWS];
+    int64_t v = x + sy * y0 + sz * z0;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        in[r] = y0 + r < ny;  // (a column past the last has no row)
+        tc[r] = in[r] ? T[v + r * sy] : 0.0;
+        kc[r] = in[r] ? klass(v + r * sy) : 0;
+        fzm[r] = in[r] ? flux(z0 > 0, 4, v + r * sy - sz, tc[r], kc[r]) : 0.0;
+    }
     unsigned errbits = 0;
     for (int z = z0; z < z1; ++z, v += sz) {
         const bool up = z + 1 < nz;
-        const double tp = up ? __ldg(T + v + sz) : 0.0;
-        const int kp = up ? klass(v + sz) : kc;
-        const double Jv = src_on ? J[v] : 0.0;
-        const double dxm = face(x > 0, 0, v - 1, tc, kc), dxp = face(x < nx - 1, 1, v + 1, tc, kc);
-        const double dym = face(y > 0, 2, v - sy, tc, kc), dyp = face(y < ny - 1, 3, v + sy, tc, kc);
-        const double dzm = z > 0 ? tm - tc : face(false, 4, 0, tc, kc);
-        const double dzp = up ? tp - tc : face(false, 5, 0, tc, kc);
-        double dT;
-        if (UNIFORM) {
-            dT = fma(Cz, dzm + dzp, fma(Cy, dym + dyp, Cx * (dxm + dxp)));
-        } else {
-            const double *f = s_fa + kc * MAX_MAT;
-            const double sx = f[x > 0 ? klass(v - 1) : kc] * dxm + f[x < nx - 1 ? klass(v + 1) : kc] * dxp;
-            const double sy_ = f[y > 0 ? klass(v - sy) : kc] * dym + f[y < ny - 1 ? klass(v + sy) : kc] * dyp;
-            const double sz_ = f[z > 0 ? km : kc] * dzm + f[kp] * dzp;
-            dT = fma(czd, sz_, fma(cyd, sy_, cxd * sx));
+        double tp[ROWS], fzp[ROWS], Jv[ROWS];
+        int kp[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const int64_t q = v + r * sy;
+            tp[r] = in[r] && up ? __ldg(T + q + sz) : 0.0;
+            kp[r] = in[r] && up ? klass(q + sz) : kc[r];
+            Jv[r] = in[r] && src_on ? J[q] : 0.0;
         }
-        double Tn = tc + (src_on ? fma(UNIFORM ? Ku : s_src[kc], Jv, dT) : dT);
-        if (ieee::bits(tc) >= boil && tc >= a.dc[FC_TBOIL]) {
-            // latent-heat clamp (src/3dFD.f90:169-175)
-            const double qv = a.dc[FC_LW] * L.rho[kc] * a.dc[FC_VVOX];
-            double *Q = (double *)a.Q;
-            const double Qv = Q[v];
-            if (Qv < qv) {
-                const double Ein = (Pdt * Jv + L.rho[kc] * L.c[kc] * dT) * a.dc[FC_VVOX];
-                if (Ein > 0.0) {
-                    const double qn = Qv + Ein;
-                    Q[v] = qn < qv ? qn : qv;
-                    Tn = a.dc[FC_TBOIL];
+        double fy = in[0] ? flux(y0 > 0, 2, v - sy, tc[0], kc[0]) : 0.0;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            if (!in[r]) continue;
+            const int64_t q = v + r * sy;
+            const double fym = fy;
+            double fyp;
+            if (r + 1 < ROWS && in[r + 1 < ROWS ? r + 1 : r]) {
+                constexpr int R1 = ROWS - 1;
+                const int rn = r < R1 ? r + 1 : R1;
+                const double d = tc[rn] - tc[r];
+                fyp = UNIFORM ? d : s_fa[kc[r] * MAX_MAT + kc[rn]] * d;
+                fy = -fyp;
+            } else {
+                fyp = flux(y0 + r < ny - 1, 3, q + sy, tc[r], kc[r]);
+            }
+            const double fxm = flux(x > 0, 0, q - 1, tc[r], kc[r]), fxp = flux(x < nx - 1, 1, q + 1, tc[r], kc[r]);
+            if (up) {
+                const double d = tp[r] - tc[r];
+                fzp[r] = UNIFORM ? d : s_fa[kc[r] * MAX_MAT + kp[r]] * d;
+            } else {
+                fzp[r] = flux(false, 5, 0, tc[r], kc[r]);
+            }
+            const double ax = UNIFORM ? Cx : cxd, ay = UNIFORM ? Cy : cyd, az = UNIFORM ? Cz : czd;
+            const double dT = fma(az, fzm[r] + fzp[r], fma(ay, fym + fyp, ax * (fxm + fxp)));
+            double Tn = tc[r] + (src_on ? fma(UNIFORM ? Ku : s_src[kc[r]], Jv[r], dT) : dT);
+            if (ieee::bits(tc[r]) >= boil && tc[r] >= a.dc[FC_TBOIL]) {
+                // latent-heat clamp (src/3dFD.f90:169-175)
+                const int k = kc[r];
+                const double qv = a.dc[FC_LW] * L.rho[k] * a.dc[FC_VVOX];
+                double *Q = (double *)a.Q;
+                const double Qv = Q[q];
+                if (Qv < qv) {
+                    const double Ein = (Pdt * Jv[r] + L.rho[k] * L.c[k] * dT) * a.dc[FC_VVOX];
+                    if (Ein > 0.0) {
+                        const double qn = Qv + Ein;
+                        Q[q] = qn < qv ? qn : qv;
+                        Tn = a.dc[FC_TBOIL];
+                    }
                 }
             }
+            To[q] = Tn;
+            if (ieee::bits(Tn) >= screen) {
+                if (ieee::is_nan(Tn)) errbits |= DEVERR_NAN;
+                else if (ieee::lt_zero(Tn)) errbits |= DEVERR_NEG_T;
+                else s_list[atomicAdd(&s_cnt, 1)] = (unsigned short)(((z - z0) * ROWS + r) * TPB64 + threadIdx.x);
+            }
+            // the next plane's z- difference
+            fzm[r] = -fzp[r];
+            tc[r] = tp[r];
+            kc[r] = kp[r];
         }
-        To[v] = Tn;
-        if (ieee::bits(Tn) >= screen) {
-            if (!(Tn == Tn)) errbits |= DEVERR_NAN;
-            else if (Tn < 0.0) errbits |= DEVERR_NEG_T;
-            else if (Tn >= a.dc[FC_SCREEN]) rare_update<double>(a, v, ni, Tn, t_new);
-        }
-        tm = tc;
-        tc = tp;
-        km = kc;
-        kc = kp;
     }
     if (errbits) atomicOr(a.err, errbits);
+    __syncthreads();
+    for (int n = threadIdx.x; n < s_cnt; n += TPB64) {
+        const int l = s_list[n], r = l / TPB64;
+        const int64_t c = col0 + l % TPB64;
+        const int64_t q = c % nx + sy * ((c / nx) * ROWS + r % ROWS) + sz * (z0 + r / ROWS);
+        rare_update<double>(a, q, ni, To[q], t_new);
+    }
 }
 
 // The class of every voxel from its k, rho, c: the first class that has them.
@@ -146,14 +193,17 @@ cudaError_t launch_cls64_step(const FusedArgs &a0, const ClassLut64 &L0, const u
     ClassLut64 L = L0;
     for (int f = 0; f < 6; ++f)
         for (int k = 0; k < MAX_MAT; ++k) L.hdk[f * MAX_MAT + k] = a.dc[FC_BCHD + f] / L.k[k];
-    const int bx = (a.nx + CX - 1) / CX, by = (a.ny + CY - 1) / CY;
-    // columns of up to 16 planes, short enough for eight blocks per SM where the grid allows
-    const int chunks = std::max(1, std::min(a.nz, (152 * 8 + bx * by - 1) / (bx * by)));
-    const int zchunk = a.zchunk > 0 ? a.zchunk : std::min(16, (a.nz + chunks - 1) / chunks);
-    const dim3 grid(bx, by, (a.nz + zchunk - 1) / zchunk);
+    const int64_t bx = ((int64_t)a.nx * ((a.ny + ROWS - 1) / ROWS) + TPB64 - 1) / TPB64;
+    // columns of 2 to ZMAX planes, two waves of the six blocks that an SM holds:
+    // blocks with many listed voxels then even out (100^3: 2 / 3 / 4 / 7 / 16
+    // planes -> 52.9 / 53.5 / 65.8 / 59.1 / 86.9 us; 60 x 50 x 55: 2 / 4 / 8
+    // planes -> 17.5 / 21.0 / 35.4 us)
+    const int chunks = (int)std::max<int64_t>(1, 152 * 6 * 2 / bx);
+    const int zchunk = a.zchunk > 0 ? std::min(ZMAX, a.zchunk) : std::min(ZMAX, std::max(2, (a.nz + chunks - 1) / chunks));
+    const dim3 grid((unsigned)bx, (a.nz + zchunk - 1) / zchunk);
     count_launch();
-    if (L.uniform >= 0) cls64_step_kernel<true><<<grid, dim3(CX, CY), 0, s>>>(a, L, cls, zchunk);
-    else cls64_step_kernel<false><<<grid, dim3(CX, CY), 0, s>>>(a, L, cls, zchunk);
+    if (L.uniform >= 0) cls64_step_kernel<true><<<grid, TPB64, 0, s>>>(a, L, cls, zchunk);
+    else cls64_step_kernel<false><<<grid, TPB64, 0, s>>>(a, L, cls, zchunk);
     return cudaGetLastError();
 }
 

@@ -2,6 +2,7 @@
 // (heat.cu: cp.async form; heat_tma.cu: TMA form).
 #pragma once
 
+#include "ieee_bits.h"
 #include "tam_device.cuh"
 #include "tam_kernels.h"
 
@@ -84,15 +85,16 @@ __device__ __noinline__ float ghost_faces(const FusedArgs &a, unsigned gm, float
 template <typename Real>
 __device__ __noinline__ void rare_update(const FusedArgs &a, int64_t v, int64_t ni, double Tt, double t_new)
 {
-    if (a.arrhenius && Tt >= a.T_lo && Tt < a.T_hi) {
+    // compares on the bit patterns (ieee_bits.h): off the FP64 pipe
+    if (a.arrhenius && ieee::le(a.T_lo, Tt) && ieee::lt(Tt, a.T_hi)) {
         const double o = a.omega[v];
         const double on = o + a.dt * exp(a.lnA - a.Ea / (a.Rgas * Tt));
         a.omega[v] = on;
 #pragma unroll
         for (int t = 0; t < 3; ++t)
-            if (o < a.thr[t] && on >= a.thr[t]) a.thres[v + t * ni] = t_new;
+            if (ieee::lt(o, a.thr[t]) && ieee::le(a.thr[t], on)) a.thres[v + t * ni] = t_new;
     }
-    if (Tt >= a.T_abl && a.mat[v] != 0) {
+    if (ieee::le(a.T_abl, Tt) && a.mat[v] != 0) {
         a.mat[v] = 0;  // optics -> air
         ((Real *)a.J)[v] = (Real)0;
         atomicAdd(a.n_ablated, 1ull);
