@@ -70,19 +70,25 @@ __device__ __forceinline__ double ref_axis(double a, double d, double tm, double
 }
 
 // Source, latent-heat clamp and physicality check of one voxel
-// (src/3dFD.f90:166-183); c: halo index, q: interior index.
-__device__ __forceinline__ void ref_update(const RefHeatArgs &a, int64_t c, int64_t q, double T, double cc,
-                                           double u_xx, double u_yy, double u_zz)
+// (src/3dFD.f90:166-183); c: halo index, q: interior index, u: the sum of the
+// three axis terms.  laserOn is 0 or 1 and most cells absorb nothing: a factor
+// 1 and a source of +0 (coeff finite) change no bit of the sum, whose T + increment is not -0
+// unless both are.
+__device__ __forceinline__ void ref_update(const RefHeatArgs &a, double laserOn, uint32_t c, uint32_t q, double T, double u)
 {
-    const double J = a.J[q];
-    const double tempIncrease = MUL(a.delt, ADD(ADD(u_xx, u_yy), u_zz));
-    const double energyIncrease =
-        ADD(MUL(MUL(MUL(a.laserOn, J), a.delt), a.vvox), MUL(MUL(cc, a.mvox), tempIncrease));
-    const double heat = ADD(ADD(T, tempIncrease), MUL(MUL(a.laserOn, a.coeff[c]), J));
-    double tn = heat;
+    const double J = a.J[q], cf = a.coeff[c];
+    const double tempIncrease = MUL(a.delt, u);
+    const double sum = ADD(T, tempIncrease);
+    double tn = sum;
+    if (ieee::bits(J) != 0 || !ieee::is_finite(cf) || ieee::is_zero(sum)) {
+        const double lc = ieee::bits(laserOn) == ieee::ONE ? cf : MUL(laserOn, cf);
+        tn = ADD(sum, MUL(lc, J));
+    }
     // compares on the bit patterns (ieee_bits.h); Q is read only at 373 K and above
     if (ieee::ge_pos(T, B_373)) {
-        const double Qv = a.Q[q];
+        const double Qv = a.Q[q], cc = a.heatcap[c];
+        const double energyIncrease =
+            ADD(MUL(MUL(MUL(laserOn, J), a.delt), a.vvox), MUL(MUL(cc, a.mvox), tempIncrease));
         if (ieee::lt(Qv, a.qvapor) && ieee::gt_zero(energyIncrease)) {
             const double qn = ADD(Qv, energyIncrease);
             a.Q[q] = ieee::lt(qn, a.qvapor) ? qn : a.qvapor;
@@ -99,18 +105,21 @@ __device__ __forceinline__ void ref_update(const RefHeatArgs &a, int64_t c, int6
 // FP32, added to the FP64 temperature in FP64 (so no compensation is
 // needed), and the FP32 copy of the result written beside it; the
 // latent-heat branch, rare, stays FP64.
-__device__ __forceinline__ void ref_update_f32(const RefHeatArgs &a, int64_t c, int64_t q, double T, float cc,
-                                               float u_xx, float u_yy, float u_zz)
+__device__ __forceinline__ void ref_update_f32(const RefHeatArgs &a, double laserOn, float laserf, uint32_t c,
+                                               uint32_t q, double T, float u)
 {
     const double J = a.J[q];
-    const float inc = (float)a.delt * ((u_xx + u_yy) + u_zz);
-    const float src = (float)a.laserOn * a.p32[3 * a.nh + c] * (float)J;
+    const float inc = a.deltf * u;
+    // (a zero needs no conversion, which would run on the FP64 pipe)
+    const float Jf = ieee::bits(J) != 0 ? (float)J : 0.f;
+    const float src = laserf * a.p32[3 * a.nh + c] * Jf;
     const double heat = T + (double)(inc + src);
     double tn = heat;
     if (ieee::ge_pos(T, B_373)) {
         const double Qv = a.Q[q];
         if (ieee::lt(Qv, a.qvapor)) {
-            const double energyIncrease = a.laserOn * J * a.delt * a.vvox + (double)cc * a.mvox * (double)inc;
+            const float cc = a.p32[2 * a.nh + c];
+            const double energyIncrease = laserOn * J * a.delt * a.vvox + (double)cc * a.mvox * (double)inc;
             if (ieee::gt_zero(energyIncrease)) {
                 const double qn = Qv + energyIncrease;
                 a.Q[q] = ieee::lt(qn, a.qvapor) ? qn : a.qvapor;
@@ -123,6 +132,15 @@ __device__ __forceinline__ void ref_update_f32(const RefHeatArgs &a, int64_t c, 
     if (ieee::is_nan(tn)) atomicOr(a.err, DEVERR_NAN);
     a.tn[c] = tn;
     a.sn[c] = (float)tn;
+}
+
+// A cell's class for the reference stencil's face coefficients.
+__device__ __forceinline__ uint8_t ref_class(const RefClasses &r, double k, double d, double c)
+{
+    auto same = [&](const double *p) {
+        return ((ieee::bits(k) ^ ieee::bits(p[0])) | (ieee::bits(d) ^ ieee::bits(p[1])) | (ieee::bits(c) ^ ieee::bits(p[2]))) == 0;
+    };
+    return same(r.skin) ? 0 : (same(r.halo) ? 1 : 2);
 }
 
 // Face terms and axis sums of the reference stencil in the working precision
@@ -153,71 +171,210 @@ template <> struct RefOps<float> {
     }
 };
 
-// The reference stencil (src/3dFD.f90:113-187) with every face coefficient
-// computed once: a face term is symmetric in its two voxels (IEEE addition
-// and multiplication commute), so a voxel's plus face is its neighbour's
-// minus face, bit for bit.  Blocks of 32 x 8 columns march REF_ZC planes:
-// the x plus face comes from the next lane (shuffle), the y plus face from
-// the next row (shared memory), the z plus face becomes the next plane's
-// minus face; only the tile's last lane, last row and last plane compute
-// theirs.  Three divisions per voxel instead of six.  F = double: the parity
-// form; F = float: the FP32 form of reference mode.
-constexpr int REF_ZC = 8;
-template <typename F> __global__ void __launch_bounds__(256) ref_stencil_kernel(const RefHeatArgs a0)
+// The reference stencil (src/3dFD.f90:113-187), F = double: the parity form;
+// F = float: the FP32 form of reference mode.
+//
+// What bounded it was the FP64 pipe (82 % busy), two thirds of it the three
+// divisions a voxel's face coefficients take.  Nearly all voxels hold the
+// properties of unheated skin, so a class per cell (RefHeatArgs::cls: unheated
+// skin, the halo as set up, anything else) tells which faces have one of two
+// known coefficients; the others are evaluated from kappa, density and heat
+// capacity as before.  Between faces with the skin coefficient g the products
+// of the axis sums are shared: g T of a cell serves its two neighbours, and
+// 2 g T its own term (an exponent increment), along z from plane to plane and
+// along y inside a row pair.  Every shortcut gives the bits of the Fortran's own
+// operations: about 17 FP64 operations per voxel against 80.  80^3: 107 -> 33 us
+// (FP64), 24 -> 15 us (FP32, which was bound by the latency of two barriers
+// per plane).  Threads take consecutive columns of the x-y plane, wrapping
+// from row pair to row pair, so no lane idles past a row's end.
+constexpr int REF_TPB = 128, REF_ROWS = 2;
+// a coefficient from the properties of its two cells (rare: kept out of line)
+template <typename F>
+__device__ __noinline__ F ref_face_at(const F *K, const F *Dn, const F *C, uint32_t p, uint32_t q, F id2)
 {
-    // the iteration's laserOn from device memory when replayed from a graph
-    RefHeatArgs a = a0;
-    if (a0.laser_dev) a.laserOn = *a0.laser_dev;
+    return RefOps<F>::face(K[p], K[q], Dn[p], Dn[q], C[p], C[q], id2);
+}
+template <typename F>
+__global__ void __launch_bounds__(REF_TPB, 4) ref_stencil_kernel(const __grid_constant__ RefHeatArgs a0, int zc)
+{
     using O = RefOps<F>;
-    __shared__ F s_fy[8][32];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i = blockIdx.x * 32 + tx + 1, j = blockIdx.y * 8 + ty + 1;
-    const bool in = i <= a.nx && j <= a.ny;
-    // lanes past the last interior cell load a halo cell (their faces are the
-    // neighbours' plus faces) or, further out, a clamped one that is never used
-    const int ic = min(i, a.nx + 1), jc = min(j, a.ny + 1);
-    const int k0 = blockIdx.z * REF_ZC + 1, k1 = min(a.nz, k0 + REF_ZC - 1);
-    const H I{a.nx + 2, a.ny + 2};
+    constexpr int R = REF_ROWS;
+    constexpr bool D = sizeof(F) == 8;
+    const RefHeatArgs &a = a0;
+    // the iteration's laserOn from device memory when replayed from a graph
+    const double laserOn = a.laser_dev ? *a.laser_dev : a.laserOn;
+    const float laserf = D ? 0.f : (float)laserOn;
+    const unsigned FULL = 0xffffffffu;
+    const int64_t col = blockIdx.x * (int64_t)REF_TPB + threadIdx.x;
+    const int i = (int)(col % a.nx) + 1, j0 = (int)(col / a.nx) * R + 1;
+    const int k0 = blockIdx.y * zc + 1, k1 = min(a.nz, k0 + zc - 1);
+    const uint32_t sy = a.nx + 2, sz = sy * (a.ny + 2), nxy = (uint32_t)a.nx * a.ny;
     // the fields the stencil reads: FP64 for the parity form, the FP32
     // copies for the precision form (whose update still adds to the FP64 T)
-    const F *K, *D, *C, *tt;
-    if constexpr (sizeof(F) == 8) {
-        K = a.kappa, D = a.density, C = a.heatcap, tt = a.t0;
+    const F *K, *Dn, *C, *tt;
+    if constexpr (D) {
+        K = a.kappa, Dn = a.density, C = a.heatcap, tt = a.t0;
     } else {
-        K = a.p32, D = a.p32 + a.nh, C = a.p32 + 2 * a.nh, tt = a.s0;
+        K = a.p32, Dn = a.p32 + a.nh, C = a.p32 + 2 * a.nh, tt = a.s0;
     }
-    const F idx2 = (F)a.idx2, idy2 = (F)a.idy2, idz2 = (F)a.idz2;
-    int64_t c = I(ic, jc, k0);
-    const int64_t sz = (int64_t)(a.nx + 2) * (a.ny + 2), sy = a.nx + 2;
-    F kc = K[c], dc = D[c], cc = C[c];
-    F fzm = O::face(kc, K[c - sz], dc, D[c - sz], cc, C[c - sz], idz2);
-    for (int k = k0; k <= k1; ++k, c += sz) {
-        const F kp = K[c + sz], dp = D[c + sz], cp = C[c + sz];
-        const F fzp = O::face(kc, kp, dc, dp, cc, cp, idz2);
-        const F fym = O::face(kc, K[c - sy], dc, D[c - sy], cc, C[c - sy], idy2);
-        const F fxm = O::face(kc, K[c - 1], dc, D[c - 1], cc, C[c - 1], idx2);
-        s_fy[ty][tx] = fym;
-        F fxp = __shfl_down_sync(0xffffffffu, fxm, 1);
-        if (tx == 31 && ic <= a.nx) fxp = O::face(kc, K[c + 1], dc, D[c + 1], cc, C[c + 1], idx2);
-        __syncthreads();
-        F fyp = 0;
-        if (ty < 7) fyp = s_fy[ty + 1][tx];
-        else if (jc <= a.ny) fyp = O::face(kc, K[c + sy], dc, D[c + sy], cc, C[c + sy], idy2);
-        __syncthreads();  // the row is read before the next plane overwrites it
-        if (in) {
-            const F t = tt[c];
-            const F u_zz = O::axis(fzm, fzp, tt[c - sz], t, tt[c + sz]);
-            const F u_yy = O::axis(fym, fyp, tt[c - sy], t, tt[c + sy]);
-            const F u_xx = O::axis(fxm, fxp, tt[c - 1], t, tt[c + 1]);
-            const int64_t q = (int64_t)(i - 1) + (int64_t)a.nx * ((int64_t)(j - 1) + (int64_t)a.ny * (int64_t)(k - 1));
-            if constexpr (sizeof(F) == 8) ref_update(a, c, q, t, cc, u_xx, u_yy, u_zz);
-            else ref_update_f32(a, c, q, a.t0[c], cc, u_xx, u_yy, u_zz);
+    const uint8_t *cls = a.cls;
+    F id2[3];
+    // face coefficients per axis: skin to skin, skin to halo
+    F gs[3], gh[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        if constexpr (D) {
+            id2[x] = x == 0 ? a.idx2 : (x == 1 ? a.idy2 : a.idz2);
+            gs[x] = a.g_skin[x];
+            gh[x] = a.g_halo[x];
+        } else {
+            // (converted on the host: a conversion runs on the FP64 pipe)
+            id2[x] = a.id2f[x];
+            gs[x] = O::face(a.skinf[0], a.skinf[0], a.skinf[1], a.skinf[1], a.skinf[2], a.skinf[2], id2[x]);
+            gh[x] = O::face(a.skinf[0], a.halof[0], a.skinf[1], a.halof[1], a.skinf[2], a.halof[2], id2[x]);
         }
-        fzm = fzp;
-        kc = kp;
-        dc = dp;
-        cc = cp;
     }
+    // the coefficient between cells p and q of classes cp and cq
+    auto face = [&](int cp, int cq, uint32_t p, uint32_t q, int x) -> F {
+        if (cp + cq > 1) {
+            if constexpr (D) return ref_face_at<F>(K, Dn, C, p, q, id2[x]);
+            else return O::face(K[p], K[q], Dn[p], Dn[q], C[p], C[q], id2[x]);
+        }
+        return cp + cq ? gh[x] : gs[x];
+    };
+    bool in[R];
+    uint32_t c[R], q[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        in[r] = j0 + r <= a.ny;
+        const int j = min(j0 + r, a.ny);  // a row past the last repeats it, unused
+        c[r] = i + sy * j + sz * k0;
+        q[r] = (i - 1) + a.nx * (j - 1) + nxy * (k0 - 1);
+    }
+    F tm[R], t[R];
+    int km[R], kc[R];
+    double pm[R], p0[R];  // D: g T of the plane below and of this one
+    F fz[R];              // else: the coefficient of the face below
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        tm[r] = tt[c[r] - sz];
+        t[r] = tt[c[r]];
+        km[r] = cls[c[r] - sz];
+        kc[r] = cls[c[r]];
+        if constexpr (D) {
+            pm[r] = MUL(gs[2], tm[r]);
+            p0[r] = MUL(gs[2], t[r]);
+        } else {
+            fz[r] = face(km[r], kc[r], c[r] - sz, c[r], 2);
+        }
+    }
+    for (int k = k0; k <= k1; ++k) {
+        F tp[R], xm[R], xp[R];
+        int kp[R], cxm[R], cxp[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            tp[r] = tt[c[r] + sz];
+            kp[r] = cls[c[r] + sz];
+            xm[r] = tt[c[r] - 1];
+            xp[r] = tt[c[r] + 1];
+            cxm[r] = cls[c[r] - 1];
+            cxp[r] = cls[c[r] + 1];
+        }
+        // the row below the pair and the row above it (above its last row inside the grid)
+        const F ym = tt[c[0] - sy], yp = tt[c[R - 1] + sy];
+        const int cym = cls[c[0] - sy], cyp = cls[c[R - 1] + sy];
+        F u[R];
+        if constexpr (D) {
+            double pp[R], uz[R], uy[R], ux[R];
+            bool zs = true, ys = (cym | cyp) == 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                pp[r] = MUL(gs[2], tp[r]);
+                zs = zs && (km[r] | kc[r] | kp[r]) == 0;
+                ys = ys && kc[r] == 0;
+            }
+            // whole warps of skin take the shared products
+            if (__all_sync(FULL, zs)) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) uz[r] = ADD(SUB(pm[r], ieee::twice_product(p0[r], gs[2], t[r])), pp[r]);
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    uz[r] = O::axis(face(km[r], kc[r], c[r] - sz, c[r], 2), face(kc[r], kp[r], c[r], c[r] + sz, 2), tm[r],
+                                    t[r], tp[r]);
+            }
+            if (__all_sync(FULL, ys && in[R - 1])) {
+                double py[R + 2];
+                py[0] = MUL(gs[1], ym);
+                py[R + 1] = MUL(gs[1], yp);
+#pragma unroll
+                for (int r = 0; r < R; ++r) py[r + 1] = MUL(gs[1], t[r]);
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    uy[r] = ADD(SUB(py[r], ieee::twice_product(py[r + 1], gs[1], t[r])), py[r + 2]);
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const bool lo = r == 0, hi = r + 1 == R || !in[r + 1 < R ? r + 1 : r];
+                    const F tl = lo ? ym : t[r > 0 ? r - 1 : 0], th = hi ? yp : t[r + 1 < R ? r + 1 : r];
+                    const int cl = lo ? cym : kc[r > 0 ? r - 1 : 0], ch = hi ? cyp : kc[r + 1 < R ? r + 1 : r];
+                    uy[r] = O::axis(face(cl, kc[r], c[r] - sy, c[r], 1), face(kc[r], ch, c[r], c[r] + sy, 1), tl, t[r], th);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (kc[r] == 0 && (cxm[r] | cxp[r]) < 2) {
+                    // 2 b of the axis sum from the two classes
+                    const double b2 = cxm[r] + cxp[r] == 0 ? a.b2x[0] : (cxm[r] + cxp[r] == 1 ? a.b2x[1] : a.b2x[2]);
+                    ux[r] = ADD(SUB(MUL(cxm[r] ? gh[0] : gs[0], xm[r]), MUL(b2, t[r])), MUL(cxp[r] ? gh[0] : gs[0], xp[r]));
+                } else {
+                    ux[r] = O::axis(face(cxm[r], kc[r], c[r] - 1, c[r], 0), face(kc[r], cxp[r], c[r], c[r] + 1, 0), xm[r],
+                                    t[r], xp[r]);
+                }
+                u[r] = ADD(ADD(ux[r], uy[r]), uz[r]);
+                pm[r] = p0[r];
+                p0[r] = pp[r];
+            }
+        } else {
+            // a face shared by two of the thread's voxels is formed once
+            F fy = face(cym, kc[0], c[0] - sy, c[0], 1);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const bool lo = r == 0, hi = r + 1 == R || !in[r + 1 < R ? r + 1 : r];
+                const F tl = lo ? ym : t[r > 0 ? r - 1 : 0], th = hi ? yp : t[r + 1 < R ? r + 1 : r];
+                const int ch = hi ? cyp : kc[r + 1 < R ? r + 1 : r];
+                const F fzp = face(kc[r], kp[r], c[r], c[r] + sz, 2), fyp = face(kc[r], ch, c[r], c[r] + sy, 1);
+                const F uz = O::axis(fz[r], fzp, tm[r], t[r], tp[r]);
+                const F uy = O::axis(fy, fyp, tl, t[r], th);
+                const F ux = O::axis(face(cxm[r], kc[r], c[r] - 1, c[r], 0), face(kc[r], cxp[r], c[r], c[r] + 1, 0), xm[r],
+                                     t[r], xp[r]);
+                fz[r] = fzp;
+                fy = fyp;
+                u[r] = (ux + uy) + uz;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (in[r]) {
+                if constexpr (D) ref_update(a, laserOn, c[r], q[r], t[r], u[r]);
+                else ref_update_f32(a, laserOn, laserf, c[r], q[r], a.t0[c[r]], u[r]);
+            }
+            tm[r] = t[r];
+            t[r] = tp[r];
+            km[r] = kc[r];
+            kc[r] = kp[r];
+            c[r] += sz;
+            q[r] += nxy;
+        }
+    }
+}
+
+// The class of every cell, halo included, from its properties.
+__global__ void ref_classes_kernel(int64_t nh, const double *kappa, const double *density, const double *heatcap,
+                                   const RefClasses r, uint8_t *cls)
+{
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nh; c += (int64_t)gridDim.x * blockDim.x)
+        cls[c] = ref_class(r, kappa[c], density[c], heatcap[c]);
 }
 
 // Arrhenius damage of one voxel: T and rk its temperature and extinction,
@@ -344,6 +501,7 @@ __device__ __forceinline__ void props_voxel(const RefPropsArgs &a, int i, int j,
         a.heatcap[c] = hc;
         a.kappa[c] = kk;
         a.coeff[c] = cf;
+        a.cls[c] = ref_class(a.classes, kk, dn, hc);
         if (a.p32) store_p32(a, c, kk, dn, hc, cf);
     } else {
         if (ieee::lt_zero(T)) atomicOr(a.err, DEVERR_NEG_T);
@@ -357,6 +515,7 @@ __device__ __forceinline__ void props_voxel(const RefPropsArgs &a, int i, int j,
         a.alpha[c] = DIV(kk, MUL(dn, hc));
         const double cf = DIV(a.delt, MUL(air_dens(T), hc));
         a.coeff[c] = cf;
+        a.cls[c] = 2;
         if (a.p32) store_p32(a, c, kk, dn, hc, cf);
     }
 }
@@ -768,12 +927,49 @@ __global__ void from_halo_kernel(const FusedArgs a, const double *halo)
 
 }  // namespace
 
-cudaError_t launch_ref_stencil(const RefHeatArgs &a, cudaStream_t s)
+void ref_class_faces(RefHeatArgs &a, const RefClasses &r)
 {
+    const double id2[3] = {a.idx2, a.idy2, a.idz2};
+    auto half = [](double x) { return 0.5 * x; };
+    for (int x = 0; x < 3; ++x) {
+        auto face = [&](const double *p, const double *q) {
+            const double kh = half(p[0] + q[0]), dh = half(p[1] + q[1]), ch = half(p[2] + q[2]);
+            const volatile double dc = dh * ch;
+            return half(kh / dc) * id2[x];
+        };
+        a.g_skin[x] = face(r.skin, r.skin);
+        a.g_halo[x] = face(r.skin, r.halo);
+    }
+    const double g[2] = {a.g_skin[0], a.g_halo[0]};
+    for (int n = 0; n < 3; ++n) a.b2x[n] = 2.0 * half(g[n > 1] + g[n > 0]);
+    for (int n = 0; n < 3; ++n) {
+        a.skinf[n] = (float)r.skin[n];
+        a.halof[n] = (float)r.halo[n];
+        a.id2f[n] = (float)id2[n];
+    }
+}
+
+cudaError_t launch_ref_classes(int64_t nh, const double *kappa, const double *density, const double *heatcap,
+                               const RefClasses &r, uint8_t *cls, cudaStream_t s)
+{
+    if (nh <= 0) return cudaSuccess;
     count_launch();
-    const dim3 grid((a.nx + 31) / 32, (a.ny + 7) / 8, (a.nz + REF_ZC - 1) / REF_ZC);
-    if (a.f32) ref_stencil_kernel<float><<<grid, dim3(32, 8), 0, s>>>(a);
-    else ref_stencil_kernel<double><<<grid, dim3(32, 8), 0, s>>>(a);
+    ref_classes_kernel<<<(unsigned)std::min<int64_t>((nh + 255) / 256, 152 * 16), 256, 0, s>>>(nh, kappa, density, heatcap, r, cls);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ref_stencil(const RefHeatArgs &a0, cudaStream_t s)
+{
+    RefHeatArgs a = a0;
+    a.deltf = (float)a.delt;
+    count_launch();
+    const int64_t bx = ((int64_t)a.nx * ((a.ny + REF_ROWS - 1) / REF_ROWS) + REF_TPB - 1) / REF_TPB;
+    // columns of 2 to 16 planes, four blocks per SM where the grid allows
+    const int chunks = (int)std::max<int64_t>(1, 152 * 4 / bx);
+    const int zc = std::min(16, std::max(2, (a.nz + chunks - 1) / chunks));
+    const dim3 grid((unsigned)bx, (a.nz + zc - 1) / zc);
+    if (a.f32) ref_stencil_kernel<float><<<grid, REF_TPB, 0, s>>>(a, zc);
+    else ref_stencil_kernel<double><<<grid, REF_TPB, 0, s>>>(a, zc);
     return cudaGetLastError();
 }
 

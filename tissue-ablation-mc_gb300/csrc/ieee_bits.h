@@ -32,6 +32,7 @@ namespace ieee {
 
 constexpr uint64_t SIGN = 0x8000000000000000ull;
 constexpr uint64_t PINF = 0x7FF0000000000000ull;  // +inf; |x| bits above this are NaN
+constexpr uint64_t ONE = 0x3FF0000000000000ull;   // 1.0
 
 TAM_HD uint64_t bits(double x)
 {
@@ -50,6 +51,8 @@ TAM_HD uint64_t bits(double x)
 
 // x != x
 TAM_HD bool is_nan(double x) { return (bits(x) & ~SIGN) > PINF; }
+// neither infinite nor NaN
+TAM_HD bool is_finite(double x) { return (bits(x) & ~SIGN) < PINF; }
 // x == 0.0 (either zero)
 TAM_HD bool is_zero(double x) { return (bits(x) << 1) == 0; }
 // x > 0.0: +min denormal .. +inf
@@ -125,6 +128,22 @@ TAM_HD double twice_half(double s, double h)
     if (((sb & ~SIGN) >> 52) >= 2u) return s;
     const uint64_t hb = bits(h);
     return from_bits((hb & SIGN) | ((hb & ~SIGN) << 1));
+}
+
+// The product (2 g) t for a g whose double does not overflow, given p = g t
+// (each rounded to nearest even), on the
+// bit pattern: twice p when p is normal and stays finite (a doubling moves no
+// significand bit, so it commutes with the rounding), else the product itself.
+TAM_HD double twice_product(double p, double g, double t)
+{
+    const uint64_t b = bits(p), e = (b >> 52) & 0x7FFu;
+    if (e - 1u < 2045u) return from_bits(b + (1ull << 52));
+#if defined(__CUDA_ARCH__)
+    return __dmul_rn(__dmul_rn(2.0, g), t);
+#else
+    const double g2 = 2.0 * g;
+    return g2 * t;
+#endif
 }
 
 }  // namespace ieee

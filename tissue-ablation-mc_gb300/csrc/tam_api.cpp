@@ -153,6 +153,11 @@ struct tam_ctx {
     bool use_slab = true;            // class-table step: the slab form where the grid allows it
     uint8_t *d_cls = nullptr;
     int cls_pitch = 0;
+    // reference mode: the cells' classes (tam_kernels.h, RefClasses); rebuilt
+    // from the properties after anything but the property update wrote them
+    tam::RefClasses rcls{};
+    uint8_t *d_rcls = nullptr;
+    bool rcls_ok = false;
     // FP64 contexts: the class tables and grid of the class-table step; the
     // grid is made from k, rho, c when a heat call first needs it
     tam::ClassLut64 clut64{};
@@ -186,6 +191,7 @@ void fields_changed(tam_ctx *ctx)
 {
     ctx->props_delt = -1.0;
     ctx->shadow_ok = false;
+    ctx->rcls_ok = false;
 }
 }  // namespace
 
@@ -394,6 +400,18 @@ int ref_setup(tam_ctx *ctx)
     CK(tam::launch_fill_halo(ctx->d_alpha, nx, ny, nz, alphatmp, alphatmp, alpha_air, true, s));
     CK(tam::launch_fill_halo(ctx->d_kappa, nx, ny, nz, skin_cond(WATER_INIT, densitytmp), air_cond(25. + 273.), 0.0,
                              false, s));
+    {
+        // unheated skin in the operations (each rounded) of the property update's kernel
+        auto mul = [](double x, double y) { volatile double r = x * y; return (double)r; };
+        auto add = [](double x, double y) { volatile double r = x + y; return (double)r; };
+        const double w = WATER_INIT, dn = 1000.0 / add(w, mul(0.649, 0.25));
+        ctx->rcls.skin[0] = mul(dn, add(mul(6.28e-4, w), mul(1.17e-4, 0.25)));
+        ctx->rcls.skin[1] = dn;
+        ctx->rcls.skin[2] = mul(1000.0, add(mul(4.2, w), mul(1.09, 0.25)));
+        ctx->rcls.halo[0] = air_cond(25. + 273.);
+        ctx->rcls.halo[1] = densitytmp;
+        ctx->rcls.halo[2] = heatCaptmp;
+    }
     CK(tam::launch_fill_f64(ctx->d_density, densitytmp, ctx->nh, s));
     CK(tam::launch_fill_f64(ctx->d_heatcap, heatCaptmp, ctx->nh, s));
     const double constd = (1.0 / (ctx->dx * ctx->dx)) + (1.0 / (ctx->dy * ctx->dy)) + (1.0 / (ctx->dz * ctx->dz));
@@ -750,6 +768,14 @@ int refresh_tallies(tam_ctx *ctx)
 }
 
 // ------------------------------------------------------ heat (reference) --
+int ref_classes(tam_ctx *ctx)
+{
+    if (ctx->rcls_ok) return TAM_OK;
+    CK(tam::launch_ref_classes(ctx->nh, ctx->d_kappa, ctx->d_density, ctx->d_heatcap, ctx->rcls, ctx->d_rcls, ctx->stream));
+    ctx->rcls_ok = true;
+    return TAM_OK;
+}
+
 int ref_heat(tam_ctx *ctx, int32_t loops)
 {
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
@@ -784,6 +810,9 @@ int ref_heat(tam_ctx *ctx, int32_t loops)
         a.p32 = ctx->d_p32;
         a.nh = ctx->nh;
     }
+    RC(ref_classes(ctx));
+    a.cls = ctx->d_rcls;
+    tam::ref_class_faces(a, ctx->rcls);
     for (int32_t it = 0; it < loops; ++it) {
         a.delt = ctx->delt;
         a.laserOn = ctx->laserOn;
@@ -841,6 +870,8 @@ tam::RefPropsArgs props_args(const tam_ctx *ctx, double ablate_temp)
     a.reuse = ctx->props_delt == ctx->delt ? 1 : 0;
     a.p32 = ctx->fp64 ? nullptr : ctx->d_p32;  // FP32 copies written beside the FP64 properties
     a.nh = ctx->nh;
+    a.cls = ctx->d_rcls;
+    a.classes = ctx->rcls;
     return a;
 }
 
@@ -1574,6 +1605,7 @@ int tam_create(const tam_params *p, const tam_config *cfg, tam_ctx **out)
         AL(ctx->d_alpha, ctx->nh);
         AL(ctx->d_Q, ctx->ni);
         AL(ctx->d_water, ctx->ni);
+        AL(ctx->d_rcls, ctx->nh);
         if (!ctx->fp64) {
             AL(ctx->d_t32[0], ctx->nh);
             AL(ctx->d_t32[1], ctx->nh);
@@ -2053,6 +2085,8 @@ bool ref_graph_capture(tam_ctx *ctx, uint64_t seed, int slot)
         h.nh = ctx->nh;
         h.delt = ctx->delt;
         h.laser_dev = &iv->laser_on;
+        h.cls = ctx->d_rcls;
+        tam::ref_class_faces(h, ctx->rcls);
         h.t0 = ctx->d_T[tcur];
         h.tn = ctx->d_T[1 - tcur];
         h.s0 = ctx->fp64 ? nullptr : ctx->d_t32[tcur];
@@ -2106,7 +2140,7 @@ int ref_run(tam_ctx *ctx, uint64_t seed, int64_t max_iters, bool until_time, int
         bool replayed = false;
         if (ctx->use_graph && ctx->ref_warm && ctx->p.loops == 1 && (it % ERR_EVERY) + G <= ERR_EVERY &&
             (max_iters <= 0 || it + G <= max_iters) && ctx->props_delt == ctx->delt && !(ctx->pulseLength < ctx->delt) &&
-            (ctx->fp64 || ctx->shadow_ok)) {
+            (ctx->fp64 || ctx->shadow_ok) && ctx->rcls_ok) {
             // run the host state ahead; roll it back if the chunk does not fit
             const double t0 = ctx->time, pc0 = ctx->pulseCount, rc0 = ctx->repetitionCount, lo0 = ctx->laserOn;
             const int lf0 = ctx->laser_flag, pf0 = ctx->pulseFlag, pd0 = ctx->pulsesDone, ll0 = ctx->loops_left;

@@ -153,6 +153,13 @@ cudaError_t launch_philox_selftest(const uint32_t *in, uint32_t *out_mine, uint3
 
 // ---------------------------------------------- reference-mode heat path --
 // Scalars of module Heat (src/3dFD.f90:7-12) needed on the device.
+// The two sets of properties (kappa, density, heat capacity) that most cells of
+// a reference-mode grid hold: skin at its initial water content, as the property
+// update evaluates it, and the halo as set up.  A cell's class is 0 or 1 if its
+// bits are those, else 2.
+struct RefClasses {
+    double skin[3], halo[3];
+};
 struct RefHeatArgs {
     int32_t nx, ny, nz;
     double idx2, idy2, idz2;          // 1/dx^2 etc (dx = 2 max 1e-2 / (n+2))
@@ -169,8 +176,17 @@ struct RefHeatArgs {
     const float *s0;                  // FP32 copy of t0
     float *sn;                        // FP32 copy of tn, written with it
     const double *laser_dev;          // non-null: laserOn is read from here
+    const uint8_t *cls;               // class of every cell (halo included), see RefClasses
+    // from the classes' properties (ref_class_faces):
+    double g_skin[3], g_halo[3];      // face coefficients per axis, skin to skin and skin to halo
+    double b2x[3];                    // 2 b of the x sum with 0, 1 or 2 halo neighbours
+    float skinf[3], halof[3], id2f[3], deltf; // FP32 form: the properties, 1/d^2 and delt in FP32
 };
+// Fills the class fields (idx2, idy2, idz2 set before).
+void ref_class_faces(RefHeatArgs &a, const RefClasses &r);
 cudaError_t launch_ref_stencil(const RefHeatArgs &a, cudaStream_t s);
+cudaError_t launch_ref_classes(int64_t nh, const double *kappa, const double *density, const double *heatcap,
+                               const RefClasses &r, uint8_t *cls, cudaStream_t s);
 
 struct RefArrheniusArgs {
     int32_t nx, ny, nz;
@@ -194,6 +210,8 @@ struct RefPropsArgs {
     int32_t reuse;                    // 1: the previous call's skin properties are intact (same delt)
     float *p32;                       // null, or FP32 copies of kappa, density, heatcap, coeff (4 x nh)
     int64_t nh;
+    uint8_t *cls;                     // classes of the cells, kept with their properties
+    RefClasses classes;
 };
 cudaError_t launch_ref_props(const RefPropsArgs &a, cudaStream_t s);
 // Arrhenius and then the property update of every voxel in one pass (their
