@@ -137,6 +137,7 @@ extern "C" int tam_mc_pass_noalloc(const tam_params *p, const double *rhokap, do
     a.jmean = acc;
     a.tally = tally;
     a.work = work;
+    a.work_zeroed = 1;
     a.err = err;
     e = tam::launch_transport(a, p->precision == TAM_FP64, sms, s);
     if (e != cudaSuccess) return fail(TAM_E_CUDA, std::string("transport: ") + cudaGetErrorString(e));

@@ -725,14 +725,17 @@ int pass_normalise(tam_ctx *ctx, int64_t n, cudaStream_t s)
     return TAM_OK;
 }
 
+// jmean, the tallies and the packet counter behind it
+size_t pass_bytes(const tam_ctx *ctx) { return ((size_t)ctx->ni + tam::N_TALLY + 1) * sizeof(double); }
+
 int mc_pass(tam_ctx *ctx, int64_t n, uint64_t seed, uint32_t stream, bool sync = true)
 {
     cudaStream_t s = ctx->stream;
     tam::TransportArgs a;
     bool t32 = false;
     RC(pass_args(ctx, n, seed, stream, a, t32));
-    CK(cudaMemsetAsync(ctx->d_jmean, 0, ctx->ni * sizeof(double), s));
-    CK(cudaMemsetAsync(ctx->d_tally, 0, tam::N_TALLY * sizeof(double), s));
+    CK(cudaMemsetAsync(ctx->d_jmean, 0, pass_bytes(ctx), s));
+    a.work_zeroed = t32 ? 0 : 1;
     CK(cudaEventRecord(ctx->ev[0], s));
     if (t32) {
         // chunks of packets with their global ids: the same Philox streams as one launch
@@ -1584,11 +1587,14 @@ int tam_create(const tam_params *p, const tam_config *cfg, tam_ctx **out)
 #define AL(ptr, n) \
     if (r == TAM_OK) r = dalloc_t(ctx, &(ptr), (n))
     AL(ctx->d_err, 1);
-    AL(ctx->d_tally, tam::N_TALLY);
-    AL(ctx->d_work, 1);
     AL(ctx->d_nabl, 1);
     AL(ctx->d_cnt, 1);
-    AL(ctx->d_jmean, ctx->ni);
+    // the pass's tallies and packet counter lie behind its tally: one memset clears all three
+    AL(ctx->d_jmean, ctx->ni + tam::N_TALLY + 1);
+    if (r == TAM_OK) {
+        ctx->d_tally = ctx->d_jmean + ctx->ni;
+        ctx->d_work = (unsigned long long *)(ctx->d_tally + tam::N_TALLY);
+    }
     AL(ctx->d_sum, 1);
     AL(ctx->d_tissue, ctx->ni);
     AL(ctx->d_thres, 3 * ctx->ni);
@@ -2057,8 +2063,8 @@ bool ref_graph_capture(tam_ctx *ctx, uint64_t seed, int slot)
         a.tally = ctx->d_tally;
         a.work = ctx->d_work;
         a.err = ctx->d_err;
-        ok = cudaMemsetAsync(ctx->d_jmean, 0, ctx->ni * sizeof(double), s) == cudaSuccess &&
-             cudaMemsetAsync(ctx->d_tally, 0, tam::N_TALLY * sizeof(double), s) == cudaSuccess &&
+        a.work_zeroed = 1;
+        ok = cudaMemsetAsync(ctx->d_jmean, 0, pass_bytes(ctx), s) == cudaSuccess &&
              tam::launch_transport(a, ctx->fp64, ctx->sm_count, s) == cudaSuccess &&
              tam::launch_scale_f64(ctx->d_jglob, ctx->d_jmean, 0.0, ctx->ni, false, s,
                                    ctx->d_tally + tam::T_ABSORBED, &iv->f) == cudaSuccess;
@@ -2378,8 +2384,7 @@ int multi_pass(TrTable &T, tam_ctx *const *ctxs, int32_t n, const std::vector<in
             for (int32_t i : grouped) {
                 tam_ctx *c = ctxs[i];
                 if (c->stream != s) CK(cudaStreamSynchronize(c->stream));
-                CK(cudaMemsetAsync(c->d_jmean, 0, c->ni * sizeof(double), s));
-                CK(cudaMemsetAsync(c->d_tally, 0, tam::N_TALLY * sizeof(double), s));
+                CK(cudaMemsetAsync(c->d_jmean, 0, pass_bytes(c), s));
             }
             CK(cudaMemcpyAsync(T.d_tr, tab.data(), sizeof(tam::BatchTrInst) * tab.size(), cudaMemcpyHostToDevice, s));
             for (int32_t i : grouped) CK(cudaEventRecord(ctxs[i]->ev[0], s));

@@ -55,6 +55,11 @@ template <typename Real> struct TrConst {
     Real namb, rhokap_n, src_r;       // ambient and rhokap-medium refractive indices, source radius
 };
 
+// One material's optics in the transport's precision.
+template <typename Real> struct MatR {
+    Real mut, mua, alb, g, g2, n;
+};
+
 struct TransportArgs {
     int32_t nx, ny, nz;
     double xmax, ymax, zmax;          // half-widths, cm
@@ -85,10 +90,14 @@ struct TransportArgs {
     int32_t bx0, by0, bz0;            // the FP32 tally's box: first cell and extent per axis
     int32_t bnx, bny, bnz;
     double *tally;                    // N_TALLY doubles
-    unsigned long long *work;         // dynamic packet counter (zeroed by the launcher)
+    unsigned long long *work;         // counter of the packets drawn after each warp's first (zeroed by the launcher
+                                      // unless work_zeroed)
+    int32_t work_zeroed;
     unsigned *err;                    // device error word
     TrConst<double> cd;               // filled by launch_transport
     TrConst<float> cf;
+    MatR<double> md[MAX_MAT];
+    MatR<float> mf[MAX_MAT];
     uint32_t rk[20];                  // Philox round keys of `seed`, filled by launch_transport
 };
 

@@ -116,22 +116,22 @@ template <typename Real> __device__ __forceinline__ const TrConst<Real> &consts(
     else return a.cd;
 }
 
+template <typename Real> __device__ __forceinline__ const MatR<Real> *mats(const TransportArgs &a)
+{
+    if constexpr (sizeof(Real) == 4) return a.mf;
+    else return a.md;
+}
+
 template <typename Real, int MED, bool T32>
 __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) transport_kernel(const __grid_constant__ TransportArgs a, int scat_min, unsigned lanes)
 {
     __shared__ MatR<Real> lut[MAX_MAT];
     __shared__ HgF hgt[sizeof(Real) == 4 ? MAX_MAT : 1];
-    for (int t = threadIdx.x; t < MAX_MAT; t += blockDim.x) {
-        const OptMat &o = a.lut[t < a.nmat ? t : 0];
-        MatR<Real> m;
-        m.mut = (Real)(o.mua + o.mus);
-        m.mua = (Real)o.mua;
-        m.alb = (o.mua + o.mus) > 0.0 ? (Real)(o.mus / (o.mua + o.mus)) : (Real)0;
-        m.g = (Real)o.g;
-        m.g2 = (Real)(o.g * o.g);
-        m.n = (Real)o.n;
-        lut[t] = m;
-        if constexpr (sizeof(Real) == 4) hgt[t] = hg_consts(m.g, m.g2);
+    if constexpr (MED != MED_RHOKAP) {
+        for (int t = threadIdx.x; t < MAX_MAT; t += blockDim.x) {
+            lut[t] = mats<Real>(a)[t];
+            if constexpr (sizeof(Real) == 4) hgt[t] = hg_consts(lut[t].g, lut[t].g2);
+        }
     }
     // per-packet (rare) tallies accumulate in shared memory, not registers
     __shared__ double s_tal[5];  // specular, reflected, transmitted, side, roulette net
@@ -152,6 +152,9 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     const Real knx = K.knx, kny = K.kny, knz = K.knz;
     const uint32_t strm = a.stream_dev ? *a.stream_dev : a.stream;
     const unsigned lane = threadIdx.x & 31u;
+    const unsigned warp_id = blockIdx.x * (TPB / 32) + (threadIdx.x >> 5), nwarps = gridDim.x * (TPB / 32);
+    const bool one_draw = (unsigned long long)nwarps * __popc(lanes) >= (unsigned long long)a.n;
+    bool first = true;
     const Real wmin = K.wmin, rm = K.rm, inv_rm = K.inv_rm;
     // weights below this need a look after a scatter: roulette, or the end of a packet without weight
     const Real w_rare = a.roulette && wmin > (Real)0 ? wmin : (Real)1.401298464e-45;
@@ -196,11 +199,16 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
         unsigned live = __ballot_sync(FULL, alive);
         const unsigned need = exhausted ? 0u : ~live & lanes;
         if (need && (__popc(need) >= TAM_REFILL_MIN || live == 0u)) {
-            const int leader = __ffs(need) - 1;
-            unsigned long long base = 0;
-            if ((int)lane == leader) base = atomicAdd(a.work, (unsigned long long)__popc(need));
-            base = __shfl_sync(FULL, base, leader);
-            exhausted = base + (unsigned long long)__popc(need) >= (unsigned long long)a.n;
+            // the first packets by the warp's place in the launch, the others
+            // from the counter of those drawn beyond them
+            unsigned long long base = first ? (unsigned long long)warp_id * __popc(lanes) : 0;
+            if (!first) {
+                const int leader = __ffs(need) - 1;
+                if ((int)lane == leader) base = atomicAdd(a.work, (unsigned long long)__popc(need));
+                base = __shfl_sync(FULL, base, leader) + (unsigned long long)nwarps * __popc(lanes);
+            }
+            first = false;
+            exhausted = base + (unsigned long long)__popc(need) >= (unsigned long long)a.n || one_draw;
             if (need >> lane & 1u) {
                 const unsigned long long my = base + __popc(need & ((1u << lane) - 1u));
                 if (my < (unsigned long long)a.n) {
@@ -258,9 +266,11 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                         nx = sint * cp;  // direction (0, 0, -1): +-0 in x and y
                         ny = sint * sp;
                         nz = (Real)-1;
-                        axis_setup(nx, fx, hx, BIG, tdx, tmx, sgx);
-                        axis_setup(ny, fy, hy, BIG, tdy, tmy, sgy);
-                        axis_setup(nz, fz, hz, BIG, tdz, tmz, sgz);
+                        // the set-up of that direction, without its divisions
+                        tdx = tdy = tmx = tmy = BIG;
+                        sgx = sgy = sgz = -1;
+                        tdz = hz;
+                        tmz = fz;
                         t = (Real)0;
                         dep = (Real)0;
                         nsteps = 0;
@@ -352,7 +362,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                         go = g != 0;
                     } else {
 #pragma unroll
-                        for (int q = 0; q < VSTEPS; ++q) vstep(std::false_type{});
+                        for (int q = 0; q < (MED == MED_RHOKAP ? 1 : VSTEPS); ++q) vstep(std::false_type{});
                     }
                 }
             } else {
@@ -581,31 +591,43 @@ __global__ void brick_table_kernel(const uint8_t *mat, int nx, int ny, int nz, i
 
 // out = in * f (normalisation of the tally), and with `sum` the total of
 // `in` added to *sum: one FP64 atomic per block, so the grid is kept to a few
-// thousand blocks
+// thousand blocks.  Most cells of a tally are zero: for a finite f >= 0 their
+// product is a zero too and they add nothing, so warps of zeros leave the
+// narrow FP64 pipe alone (it bounded this pass; 512,000 cells, few of them lit:
+// 8.6 -> 5 us).
 template <typename Out>
 __global__ void scale_kernel(Out *out, double *in, double f, int64_t n, int zero_in, double *sum,
                              const double *f_dev)
 {
     if (f_dev) f = *f_dev;
+    const bool plain = ieee::is_finite(f) && ieee::ge_zero(f);
     double acc = 0.0;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
         const double v = in[q];
+        if (plain && ieee::bits(v) == 0) {
+            out[q] = (Out)0;
+            continue;
+        }
         out[q] = (Out)(v * f);
         acc += v;
         if (zero_in) in[q] = 0.0;
     }
     if (!sum) return;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     __shared__ double ws[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (__any_sync(0xffffffffu, ieee::bits(acc) != 0)) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    }
     if (lane == 0) ws[wid] = acc;
     __syncthreads();
     if (wid == 0) {
         acc = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0.0;
+        if (__any_sync(0xffffffffu, ieee::bits(acc) != 0)) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) atomicAdd(sum, acc);
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) atomicAdd(sum, acc);
+        }
     }
 }
 
@@ -688,6 +710,12 @@ static void fill_consts(TransportArgs &a)
     d.namb = a.n_ambient;
     d.rhokap_n = a.rhokap_n;
     d.src_r = a.source_radius;
+    for (int t = 0; t < MAX_MAT; ++t) {
+        const OptMat &o = a.lut[t < a.nmat ? t : 0];
+        const double mut = o.mua + o.mus, alb = mut > 0.0 ? o.mus / mut : 0.0, g2 = o.g * o.g;
+        a.md[t] = MatR<double>{mut, o.mua, alb, o.g, g2, o.n};
+        a.mf[t] = MatR<float>{(float)mut, (float)o.mua, (float)alb, (float)o.g, (float)g2, (float)o.n};
+    }
     TrConst<float> &f = a.cf;
     f.hx = (float)d.hx, f.hy = (float)d.hy, f.hz = (float)d.hz;
     f.knx = (float)d.knx, f.kny = (float)d.kny, f.knz = (float)d.knz;
@@ -729,8 +757,10 @@ cudaError_t launch_transport(const TransportArgs &args, bool fp64, int sm_count,
     TransportArgs a = args;
     fill_consts(a);
     philox_round_keys(a.seed, a.rk);
-    cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
+    if (!a.work_zeroed) {
+        cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s);
+        if (e != cudaSuccess) return e;
+    }
     if (fp64) {
         // the FP32 box tally is a config-mode form; on the FP64 transport it
         // serves its checks against the FP64 oracle on the same streams

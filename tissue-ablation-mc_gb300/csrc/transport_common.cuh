@@ -12,10 +12,6 @@
 namespace tam {
 namespace {
 
-template <typename Real> struct MatR {
-    Real mut, mua, alb, g, g2, n;
-};
-
 // HG deflection with the arithmetic of src/stokes.f90:6-153 (PI/TWOPI are
 // the truncated constants of src/constants.f90:13).  Leaves the direction
 // unchanged when the sampled cosine is exactly +-1 (the `goto 100`).
