@@ -532,14 +532,24 @@ __global__ void ref_props_kernel(const RefPropsArgs a)
     props_voxel(a, i, j, k, c, q, a.temp[c]);
 }
 
+// A voxel that may change (out of line, so that none of its FP64 work is issued,
+// predicated off, for the others)
+__device__ __noinline__ void damage_props_voxel(const RefArrheniusArgs &d, const RefPropsArgs &a, int i, int j, int k,
+                                                uint32_t c, uint32_t q, double T, double rk)
+{
+    arrhenius_voxel(d, q, T, rk);
+    props_voxel(a, i, j, k, c, q, T);
+}
+
 // Arrhenius then the property update, voxel by voxel: the coupled loop's
 // order, one read of T and rhokap for both.  Nearly every voxel is tissue below
 // the damage window with no latent heat taken up and its initial water: nothing
 // of it changes but the ping-pong copy of rhokap.  A few integer tests decide
 // that (the general path's compares took 360 instructions per warp; 80^3:
-// 14 -> 8 us).  Threads take consecutive cells of a plane, wrapping from row to
+// 14 -> 9.8 us).  Threads take consecutive cells of a plane, wrapping from row to
 // row.
-__global__ void __launch_bounds__(256) ref_damage_props_kernel(const RefArrheniusArgs d, const RefPropsArgs a)
+__global__ void __launch_bounds__(256) ref_damage_props_kernel(const __grid_constant__ RefArrheniusArgs d,
+                                                               const __grid_constant__ RefPropsArgs a)
 {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nxy = (uint32_t)a.nx * a.ny;
@@ -560,8 +570,7 @@ __global__ void __launch_bounds__(256) ref_damage_props_kernel(const RefArrheniu
             a.rk_new[c] = rk;
             continue;
         }
-        arrhenius_voxel(d, q, T, rk);
-        props_voxel(a, i, j, k, c, q, T);
+        damage_props_voxel(d, a, i, j, k, c, q, T, rk);
     }
 }
 

@@ -12,7 +12,7 @@
 // are looked up (face coefficients per class pair, computed on the host with
 // the same means), dt is folded into them, and screens are integer compares
 // of the bit patterns: 13 FP64 operations per voxel in one class, 18 in
-// several.  100^3 cube with a core in the damage window: 443 -> 54 us per step
+// several.  100^3 cube with a core in the damage window: 443 -> 47 us per step
 // (FP64 pipe 76 % busy; a third of its operations are the window's).
 #include <algorithm>
 
@@ -26,6 +26,29 @@ namespace {
 constexpr int TPB64 = 128;
 constexpr int ROWS = 2;  // y-adjacent voxels of a thread
 constexpr int ZMAX = 16;  // planes per block at most (the list holds every voxel of a block)
+
+// The rare parts of a voxel's update, out of line: predicated off they would
+// still be issued to the FP64 pipe for every voxel (the ghosts of the six faces
+// alone were a third of its operations).
+__device__ __noinline__ double robin_diff(const FusedArgs &a, const ClassLut64 &L, int f, int k, double tc)
+{
+    return -L.hdk[f * MAX_MAT + k] * (tc - a.dc[FC_BCTA + f]);
+}
+// Latent-heat clamp (src/3dFD.f90:169-175) of a voxel that was at boiling: its new temperature.
+__device__ __noinline__ double boil64(const FusedArgs &a, const ClassLut64 &L, int k, int64_t q, double tc, double Tn,
+                                      double PJdt, double dT)
+{
+    if (!(tc >= a.dc[FC_TBOIL])) return Tn;
+    const double qv = a.dc[FC_LW] * L.rho[k] * a.dc[FC_VVOX];
+    double *Q = (double *)a.Q;
+    const double Qv = Q[q];
+    if (!(Qv < qv)) return Tn;
+    const double Ein = (PJdt + L.rho[k] * L.c[k] * dT) * a.dc[FC_VVOX];
+    if (!(Ein > 0.0)) return Tn;
+    const double qn = Qv + Ein;
+    Q[q] = qn < qv ? qn : qv;
+    return a.dc[FC_TBOIL];
+}
 
 // A thread marches ROWS y-adjacent columns through zchunk planes; the threads
 // of a block take consecutive columns of the x-y plane (x fastest, wrapping from
@@ -72,9 +95,8 @@ __global__ void __launch_bounds__(TPB64) cls64_step_kernel(const __grid_constant
     // (Dirichlet: the face's temperature; Robin: -h d / k (T - T_amb)); in a
     // grid of several classes times the face's diffusivity
     auto flux = [&](bool inside, int f, int64_t n, double tc, int k) -> double {
-        double d;
-        if (!inside && a.bc_type[f] == BC_ROBIN) d = -L.hdk[f * MAX_MAT + k] * (tc - a.dc[FC_BCTA + f]);
-        else d = (inside ? __ldg(T + n) : a.dc[FC_BCT + f]) - tc;
+        double d = (inside ? __ldg(T + n) : a.dc[FC_BCT + f]) - tc;
+        if (!inside && a.bc_type[f] == BC_ROBIN) d = robin_diff(a, L, f, k, tc);
         return UNIFORM ? d : s_fa[k * MAX_MAT + (inside ? klass(n) : k)] * d;
     };
     double tc[ROWS], fzm[ROWS];
@@ -126,21 +148,7 @@ __global__ void __launch_bounds__(TPB64) cls64_step_kernel(const __grid_constant
             const double ax = UNIFORM ? Cx : cxd, ay = UNIFORM ? Cy : cyd, az = UNIFORM ? Cz : czd;
             const double dT = fma(az, fzm[r] + fzp[r], fma(ay, fym + fyp, ax * (fxm + fxp)));
             double Tn = tc[r] + (src_on ? fma(UNIFORM ? Ku : s_src[kc[r]], Jv[r], dT) : dT);
-            if (ieee::bits(tc[r]) >= boil && tc[r] >= a.dc[FC_TBOIL]) {
-                // latent-heat clamp (src/3dFD.f90:169-175)
-                const int k = kc[r];
-                const double qv = a.dc[FC_LW] * L.rho[k] * a.dc[FC_VVOX];
-                double *Q = (double *)a.Q;
-                const double Qv = Q[q];
-                if (Qv < qv) {
-                    const double Ein = (Pdt * Jv[r] + L.rho[k] * L.c[k] * dT) * a.dc[FC_VVOX];
-                    if (Ein > 0.0) {
-                        const double qn = Qv + Ein;
-                        Q[q] = qn < qv ? qn : qv;
-                        Tn = a.dc[FC_TBOIL];
-                    }
-                }
-            }
+            if (ieee::bits(tc[r]) >= boil) Tn = boil64(a, L, kc[r], q, tc[r], Tn, Pdt * Jv[r], dT);
             To[q] = Tn;
             if (ieee::bits(Tn) >= screen) {
                 if (ieee::is_nan(Tn)) errbits |= DEVERR_NAN;
@@ -196,8 +204,8 @@ cudaError_t launch_cls64_step(const FusedArgs &a0, const ClassLut64 &L0, const u
     const int64_t bx = ((int64_t)a.nx * ((a.ny + ROWS - 1) / ROWS) + TPB64 - 1) / TPB64;
     // columns of 2 to ZMAX planes, two waves of the six blocks that an SM holds:
     // blocks with many listed voxels then even out (100^3: 2 / 3 / 4 / 7 / 16
-    // planes -> 52.9 / 53.5 / 65.8 / 59.1 / 86.9 us; 60 x 50 x 55: 2 / 4 / 8
-    // planes -> 17.5 / 21.0 / 35.4 us)
+    // planes -> 46.6 / 46.3 / 56.6 / 53.1 / 78.9 us; 60 x 50 x 55: 2 / 4 / 8
+    // planes -> 16.5 / 20.1 / 33.8 us)
     const int chunks = (int)std::max<int64_t>(1, 152 * 6 * 2 / bx);
     const int zchunk = a.zchunk > 0 ? std::min(ZMAX, a.zchunk) : std::min(ZMAX, std::max(2, (a.nz + chunks - 1) / chunks));
     const dim3 grid((unsigned)bx, (a.nz + zchunk - 1) / zchunk);

@@ -38,10 +38,11 @@ TAM_HD uint64_t bits(double x)
 {
 #if defined(__CUDA_ARCH__)
     // an opaque move: the compiler would otherwise fold the integer tests
-    // below back into FP64 compares
-    uint64_t b;
-    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
-    return b;
+    // below back into FP64 compares.  (Into two halves: as one 64-bit move of a
+    // kernel parameter it ran on the FP64 pipe.)
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+    return (uint64_t)hi << 32 | lo;
 #else
     uint64_t b;
     std::memcpy(&b, &x, sizeof b);
