@@ -340,7 +340,7 @@ def run_gpu(args):
         vb = edge ** 3
         big = {
             "workload": f"{edge}^3 homogeneous cube (2 W beam, 1e6-packet source), {nbig} heat steps after 32",
-            "kernel": "slab_step_kernel<uniform>",
+            "kernel": "quad_step_kernel<one class>",
             "us_per_step": hb * 1e3 / nbig,
             "voxel_updates_per_s": vb * nbig / (hb * 1e-3),
             "achieved": B_STENCIL_CLS * vb * nbig / (hb * 1e-3) / 1e9,
@@ -416,7 +416,7 @@ def run_gpu(args):
         },
         "roofline_stencil": {
             "bound": "hbm",
-            "kernel": "slab_step_kernel<uniform> (FP32 + Kahan, class-table coefficients, slab form)",
+            "kernel": "quad_step_kernel<one class> (FP32 + Kahan, class-table coefficients, quad form)",
             "achieved": B_STENCIL_CLS * nvox * nsteps / (heat_ms * 1e-3) / 1e9,
             "peak": hbm,
             "unit": "GB/s",

@@ -296,20 +296,19 @@ int tam_get_timing(struct tam_ctx *ctx, double *transport_ms, double *heat_ms, i
  * the grid itself inside mixed bricks -- for grids of 2^25 voxels or more, 0
  * never, 1 always; same walks either way), "heat.zchunk" (z planes per
  * thread column of the fused step, 0 = automatic; on a grid of several
- * thermal classes a change rebuilds the slab form's lists of one-class and
- * mixed blocks and synchronises the context's stream), "heat.tma" (1: stage the
+ * thermal classes the next heat call rebuilds the quad form's class table),
+ * "heat.tma" (1: stage the
  * FP32 fused step's planes with TMA where the row pitch allows, 0: cp.async),
  * "heat.cls" (1: while the thermal properties are those of the material
  * classes, look the face coefficients up per class pair instead of reading
  * per-voxel coefficient arrays; 0: always read the arrays; with TMA off or
  * rows whose pitch TMA cannot take (nx not a multiple of 4) the class-table
  * step stages its planes with cp.async, two voxels per thread),
- * "heat.slab" (class-table step with TMA: 1 (default) runs the slab form --
- * tiles of 32 x 8 voxels, two x-adjacent voxels per thread, one block
- * barrier per plane, boundary faces as ghost neighbours, boiling, damage and
- * ablation done for the listed voxels after the planes; 0 runs the form
- * chosen by "heat.cls_rows"),
- * "heat.cls_rows" (class-table step without the slab form: 0 = two
+ * "heat.slab" (class-table step with TMA: 1 (default) runs the quad form --
+ * four x-adjacent voxels per thread, boundary faces as ghost neighbours,
+ * boiling, damage and ablation done for the listed voxels after the planes;
+ * 0 runs the form chosen by "heat.cls_rows"),
+ * "heat.cls_rows" (class-table step without the quad form: 0 = two
  * x-adjacent voxels per thread; 1 or 2 = that many voxel rows per thread),
  * "heat.graph" (config mode: 1 (default) replays chunks of 16 heat steps from
  * CUDA graphs when no step but a chunk's last needs the host (re-trace check,

@@ -4,8 +4,7 @@
 // batch.cu: per step the resident blocks share out the work items (instance,
 // 32 x 8 tile, z-chunk) of every instance, and a
 // bounded software grid barrier separates the steps.  Each item is updated
-// with the scheme of the single-instance slab kernel (heat_slab.cu): two
-// x-adjacent voxels per thread, z neighbours in registers, the ghost
+// with two x-adjacent voxels per thread, z neighbours in registers, the ghost
 // neighbour of a boundary face written into the thread's own halo cell,
 // voxels needing rare work (boiling, damage window, ablation, negative or NaN)
 // listed and handled after the item's planes.  The list holds every voxel of
@@ -70,7 +69,7 @@ struct __align__(16) BItem {
 };
 
 // The listed voxels of an item whose tile starts at (bxW, byR, zb) (the
-// block's own plane stores come first), as in the single-instance slab
+// block's own plane stores come first), as in the single-instance
 // kernel: the damage-window voxels' pairs and damage integrals loaded four
 // entries at a time, the others through slab_fix; returns error bits.  The
 // whole block shares the list out, so a hot region's many entries do not

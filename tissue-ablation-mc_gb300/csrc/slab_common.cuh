@@ -1,6 +1,5 @@
-// slab_common.cuh -- per-voxel pieces of the slab-form FP32 heat step shared
-// by the single-instance kernel (heat_slab.cu) and the batched one
-// (batch_slab.cu): the fix-up of a listed voxel and the ghost neighbour of a
+// slab_common.cuh -- per-voxel pieces of the FP32 heat step shared by the
+// single-instance kernel (heat_quad.cu) and the batched one (batch_slab.cu): the fix-up of a listed voxel and the ghost neighbour of a
 // boundary face.
 #pragma once
 

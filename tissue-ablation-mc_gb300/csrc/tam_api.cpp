@@ -149,8 +149,12 @@ struct tam_ctx {
     tam::BatchInst h_sinst{};
     int s_items = 0;
     tam::FusedCls *fcls = nullptr;
-    tam::FusedSlab *fslab = nullptr;
-    bool use_slab = true;            // class-table step: the slab form where the grid allows it
+    // quad form of the class-table step: the quads' table on a heterogeneous
+    // grid, made when a heat call finds it out of date
+    bool quad = false;
+    uint8_t *d_qs = nullptr;
+    bool qs_ok = false;
+    bool use_slab = true;            // class-table step: the quad form where the grid allows it
     uint8_t *d_cls = nullptr;
     int cls_pitch = 0;
     // reference mode: the cells' classes (tam_kernels.h, RefClasses); rebuilt
@@ -471,7 +475,7 @@ int set_thermal_classes(tam_ctx *ctx, int u)
     ctx->cls64_ok = false;
     if (ctx->d_cls)
         CK(tam::launch_cls_from_mat(ctx->d_mat, nm, ctx->d_cls, ctx->nx, ctx->ny, ctx->nz, ctx->cls_pitch, ctx->stream));
-    if (ctx->d_cls && ctx->fslab && u < 0) CK(tam::fused_slab_tile_flags(ctx->fslab, ctx->zchunk, ctx->stream));
+    ctx->qs_ok = false;
     return TAM_OK;
 }
 
@@ -961,12 +965,19 @@ int staged_setup(tam_ctx *ctx)
     return TAM_OK;
 }
 
-// The slab form's per-block lists of a heterogeneous grid, for the context's
-// z-chunk (after a change of the z-chunk; synchronises the stream).
-int slab_lists(tam_ctx *ctx)
+// The quad form's table of a heterogeneous grid.
+int quad_classes(tam_ctx *ctx)
 {
-    if (!ctx->config || !ctx->d_cls || !ctx->fslab || ctx->cls_uniform >= 0) return TAM_OK;
-    CK(tam::fused_slab_tile_flags(ctx->fslab, ctx->zchunk, ctx->stream));
+    if (!ctx->quad || ctx->cls_uniform >= 0 || ctx->qs_ok) return TAM_OK;
+    if (!ctx->d_qs && dalloc_t(ctx, &ctx->d_qs, tam::quad_class_bytes(ctx->nx, ctx->ny, ctx->nz)) != TAM_OK) {
+        ctx->d_qs = nullptr;
+        ctx->quad = false;
+        ctx->err.clear();
+        return TAM_OK;
+    }
+    CK(tam::launch_quad_classes(ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->nx, ctx->ny, ctx->nz, ctx->zchunk, ctx->d_qs,
+                                ctx->stream));
+    ctx->qs_ok = true;
     return TAM_OK;
 }
 
@@ -988,11 +999,11 @@ int cls64_setup(tam_ctx *ctx)
 }
 
 // Forms of the config-mode heat step, by what the context's state allows.
-enum HeatForm { HF_CLS = 0, HF_STAGED, HF_TMA, HF_CPASYNC, HF_SLAB, HF_CLS64 };
+enum HeatForm { HF_CLS = 0, HF_STAGED, HF_TMA, HF_CPASYNC, HF_QUAD, HF_CLS64 };
 
 HeatForm heat_form(const tam_ctx *ctx)
 {
-    if (ctx->fslab && ctx->use_slab && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class) return HF_SLAB;
+    if (ctx->quad && ctx->use_slab && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class) return HF_QUAD;
     if (ctx->fcls && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class) return HF_CLS;
     if (!ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && ctx->d_cls) return HF_STAGED;
     if (ctx->tma && ctx->use_tma) return HF_TMA;
@@ -1008,7 +1019,7 @@ int launch_heat(tam_ctx *ctx, tam::FusedArgs &a, HeatForm form, int which, cudaS
     a.Tc_in = ctx->fp64 ? nullptr : ctx->d_Tc[which];
     a.Tc_out = ctx->fp64 ? nullptr : ctx->d_Tc[1 - which];
     switch (form) {
-    case HF_SLAB: CK(tam::launch_fused_slab(a, ctx->fslab, which, ctx->clut, s)); break;
+    case HF_QUAD: CK(tam::launch_quad_step(a, ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->d_qs, s)); break;
     case HF_CLS: CK(tam::launch_fused_cls(a, ctx->fcls, which, ctx->clut, ctx->cls_rows, s)); break;
     case HF_STAGED: {
         tam::BatchStep st{};
@@ -1041,8 +1052,7 @@ std::vector<unsigned char> graph_key(const tam_ctx *ctx, const tam::FusedArgs &a
     a.T_in = a.T_out = nullptr;
     a.Tc_in = nullptr;
     a.Tc_out = nullptr;
-    const int knobs[5] = {(int)form, ctx->cls_rows, ctx->zchunk, ctx->arr_fp64 ? 1 : 0,
-                          (int)tam::fused_slab_generation(ctx->fslab)};  // the slab form's block lists
+    const int knobs[4] = {(int)form, ctx->cls_rows, ctx->zchunk, ctx->arr_fp64 ? 1 : 0};
     std::vector<unsigned char> k(sizeof a + sizeof ctx->clut + sizeof knobs + 2 * sizeof(void *));
     unsigned char *p = k.data();
     std::memcpy(p, &a, sizeof a);
@@ -1051,7 +1061,7 @@ std::vector<unsigned char> graph_key(const tam_ctx *ctx, const tam::FusedArgs &a
     p += sizeof ctx->clut;
     std::memcpy(p, knobs, sizeof knobs);
     p += sizeof knobs;
-    const void *maps = form == HF_SLAB ? (const void *)ctx->fslab : (const void *)ctx->fcls;
+    const void *maps = ctx->fcls;
     std::memcpy(p, &maps, sizeof(void *));
     std::memcpy(p + sizeof(void *), &ctx->tma, sizeof(void *));
     return k;
@@ -1107,6 +1117,7 @@ int cfg_heat(tam_ctx *ctx, int32_t nsteps, int32_t *done = nullptr, bool stop_on
     tam::FusedArgs a = fused_args(ctx);
     const int check = ctx->cfg.retrace_check > 0 ? ctx->cfg.retrace_check : (stop_on_trace ? 1 : 0);
     if (nsteps > 0) RC(cls64_setup(ctx));
+    if (heat_form(ctx) == HF_QUAD && nsteps > 0) RC(quad_classes(ctx));
     const HeatForm form = heat_form(ctx);
     if (form == HF_STAGED && nsteps > 0) RC(staged_setup(ctx));
     if (form == HF_TMA && ctx->coeff_dirty && nsteps > 0) {
@@ -1664,12 +1675,7 @@ int tam_create(const tam_params *p, const tam_config *cfg, tam_ctx **out)
             (void)cudaGetLastError();
             ctx->fcls = nullptr;
         }
-        if (tam::fused_slab_supported(ctx->nx, ctx->ny, ctx->nz) &&
-            tam::fused_slab_create(&ctx->fslab, ctx->nx, ctx->ny, ctx->nz, T2, E2, (const float *)ctx->d_J,
-                                   ctx->d_cls, ctx->cls_pitch) != cudaSuccess) {
-            (void)cudaGetLastError();
-            ctx->fslab = nullptr;
-        }
+        ctx->quad = tam::quad_step_supported(ctx->nx, ctx->ny, ctx->nz);
     }
     r = ctx->config ? cfg_setup(ctx) : ref_setup(ctx);
     if (r == TAM_OK) r = finish(ctx, "tam_create");
@@ -1691,7 +1697,6 @@ int tam_destroy(tam_ctx *ctx)
         if (e) cudaEventDestroy(e);
     if (ctx->tma) tam::fused_tma_destroy(ctx->tma);
     if (ctx->fcls) tam::fused_cls_destroy(ctx->fcls);
-    if (ctx->fslab) tam::fused_slab_destroy(ctx->fslab);
     for (cudaGraphExec_t &g : ctx->gexec)
         if (g) cudaGraphExecDestroy(g);
     for (cudaGraphExec_t &g : ctx->rexec)
@@ -2934,8 +2939,7 @@ int tam_set_tuning(tam_ctx *ctx, const char *key, int64_t value)
     } else if (k == "heat.zchunk") {
         if (value < 0 || value > ctx->nz) return fail(ctx, TAM_E_INVALID, "heat.zchunk must be in 0..nz");
         ctx->zchunk = (int)value;
-        CK(cudaSetDevice(ctx->device));
-        RC(slab_lists(ctx));
+        ctx->qs_ok = false;
     } else {
         return fail(ctx, TAM_E_INVALID, "unknown tuning key " + k);
     }
@@ -3126,9 +3130,7 @@ int tam_load_state(tam_ctx *ctx, const char *path)
         if (!f) return fail(ctx, TAM_E_PARSE, "state file truncated");
         CK(cudaMemcpy(b.first, host.data(), n, cudaMemcpyHostToDevice));
     }
-    // the slab form's tile flags follow the class grid just loaded
-    if (ctx->config && ctx->d_cls && ctx->fslab && ctx->cls_uniform < 0)
-        CK(tam::fused_slab_tile_flags(ctx->fslab, ctx->zchunk, ctx->stream));
+    ctx->qs_ok = false;  // follows the class grid just loaded
     set_scalars(ctx, S);
     std::memcpy(ctx->tally, tally, sizeof tally);
     ctx->tally_stale = false;
@@ -3242,7 +3244,7 @@ int tam_autotune(tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, 
         ctx->use_slab = slab0;
         (void)cudaGetLastError();
         (void)snap_restore(ctx, S);
-        (void)slab_lists(ctx);
+        ctx->qs_ok = false;
         return code;
     };
     auto timed = [&](int ev0, int ev1) -> int {
@@ -3269,22 +3271,22 @@ int tam_autotune(tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, 
         if ((r = snap_restore(ctx, S)) != TAM_OK) return undo(r);
     }
     // heat: z planes per thread column, and the form of the class-table step
-    // (slab form, voxel pairs or rows of voxels)
+    // (quad form, voxel pairs or rows of voxels)
     if (steps > 0) {
         int best_z = ctx->zchunk, best_r = ctx->cls_rows;
         bool best_s = ctx->use_slab;
         float best_ms = 1e30f;
         const bool cls = ctx->fcls && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class;
-        const bool slab = ctx->fslab && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class;
+        const bool slab = ctx->quad && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class;
         const bool staged = !cls && !slab && !ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && ctx->d_cls;
         const std::vector<int> zcs = staged ? std::vector<int>{4, 8, 16, 32} : std::vector<int>{2, 3, 4, 5, 8, 16};
-        for (int form : {2, 0, 1}) {  // 2: slab form; 0 / 1: class-table voxel pairs / rows
+        for (int form : {2, 0, 1}) {  // 2: quad form; 0 / 1: class-table voxel pairs / rows
             if (form == 2 && !slab) continue;
             if (form == 0 && !cls) continue;
             for (int zc : zcs) {
                 if (zc > ctx->nz) continue;
                 ctx->zchunk = zc;
-                if ((r = slab_lists(ctx)) != TAM_OK) return undo(r);
+                ctx->qs_ok = false;
                 ctx->use_slab = form == 2;
                 if (form != 2) ctx->cls_rows = form;
                 if ((r = cfg_heat(ctx, steps)) != TAM_OK || (r = timed(2, 3)) != TAM_OK ||
@@ -3299,7 +3301,7 @@ int tam_autotune(tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, 
             }
         }
         ctx->zchunk = best_z;
-        if ((r = slab_lists(ctx)) != TAM_OK) return undo(r);
+        ctx->qs_ok = false;
         ctx->cls_rows = best_r;
         ctx->use_slab = best_s;
     }

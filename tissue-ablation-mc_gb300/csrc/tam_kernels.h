@@ -343,27 +343,19 @@ void fused_cls_destroy(FusedCls *m);
 cudaError_t launch_fused_cls(const FusedArgs &a, const FusedCls *m, int which, const ClassLut &L, int rows,
                              cudaStream_t s);
 
-// Slab form of the FP32 class-table step (heat_slab.cu): tiles of 32 x 8
-// voxels, voxel pairs, one block barrier per plane, boundary faces as ghost
-// neighbours in the staged planes, rare voxels (boiling, damage window,
-// ablation) redone from a per-block list after the planes.  Same layout
-// requirements as the class-table form (nx a multiple of 4, class rows of a
-// 16-byte pitch) and fewer than 2^31 voxels.
-struct FusedSlab;  // opaque: tensor maps of T[2], Tc[2], J and the class grid
-bool fused_slab_supported(int nx, int ny, int nz);
-cudaError_t fused_slab_create(FusedSlab **out, int nx, int ny, int nz, float *const T[2], float *const Tc[2],
-                              const float *J, const uint8_t *cls, int pitch);
-void fused_slab_destroy(FusedSlab *m);
-// Heterogeneous grids: recompute the slab form's per-(tile, plane) one-class
-// flags from the class grid given at creation and, for the launch at
-// `zchunk`, the lists of blocks whose tile, rim and planes hold one class
-// (run by the one-class kernel with that class) and of the others (the class
-// kernel).  Call after every change of the class grid or of the z-chunk;
-// synchronises the stream.  Without lists for the launch's z-chunk the class
-// kernel takes every block.  fused_slab_generation counts the rebuilds.
-cudaError_t fused_slab_tile_flags(FusedSlab *m, int zchunk, cudaStream_t s);
-unsigned fused_slab_generation(const FusedSlab *m);
-cudaError_t launch_fused_slab(const FusedArgs &a, const FusedSlab *m, int which, const ClassLut &L, cudaStream_t s);
+// Quad form of the FP32 class-table step (heat_quad.cu): grids whose rows are
+// whole 16-byte quads and that hold fewer than 2^31 voxels.
+bool quad_step_supported(int nx, int ny, int nz);
+// Heterogeneous grids: the update that each quad's classes ask for.  Where a 32 x 8
+// tile, its x / y rim and a run of planes (heat.zchunk of them, 6 by default, at
+// most 8, and the planes beside them) hold one class, that is the one-class
+// update.  qs: quad_class_bytes.
+int64_t quad_class_bytes(int nx, int ny, int nz);
+cudaError_t launch_quad_classes(const ClassLut &L, const uint8_t *cls, int pitch, int nx, int ny, int nz, int zchunk,
+                                uint8_t *qs, cudaStream_t s);
+// One step, as a programmatic dependent of the launch before it.
+cudaError_t launch_quad_step(const FusedArgs &a, const ClassLut &L, const uint8_t *cls, int cpitch, const uint8_t *qs,
+                             cudaStream_t s);
 
 // Batched FP32 heat step of many instances in one persistent cooperative
 // launch (batch.cu).  BatchInst lives in device memory, one per instance.
