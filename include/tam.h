@@ -297,13 +297,13 @@ int tam_get_timing(struct tam_ctx *ctx, double *transport_ms, double *heat_ms, i
  * never, 1 always; same walks either way), "heat.zchunk" (z planes per
  * thread column of the fused step, 0 = automatic; on a grid of several
  * thermal classes the next heat call rebuilds the quad form's class table),
- * "heat.tma" (1: stage the
- * FP32 fused step's planes with TMA where the row pitch allows, 0: cp.async),
+ * "heat.tma" (1: stage the FP32 fused step's planes with TMA, or run the quad
+ * form, where the row pitch allows; 0: the line form, or cp.async),
  * "heat.cls" (1: while the thermal properties are those of the material
  * classes, look the face coefficients up per class pair instead of reading
  * per-voxel coefficient arrays; 0: always read the arrays; with TMA off or
  * rows whose pitch TMA cannot take (nx not a multiple of 4) the class-table
- * step stages its planes with cp.async, two voxels per thread),
+ * step runs its line form, consecutive voxels across the rows),
  * "heat.slab" (class-table step with TMA: 1 (default) runs the quad form --
  * four x-adjacent voxels per thread, boundary faces as ghost neighbours,
  * boiling, damage and ablation done for the listed voxels after the planes;

@@ -16,8 +16,7 @@
 // "batch.staged": the default stages each tile's planes in shared memory with
 // 4-byte cp.async copies (any row pitch: the instances' edges need not be
 // multiples of four) and updates two x-adjacent voxels per thread
-// (batch_pairs_kernel, whose one-step form also serves single contexts with
-// such rows); batch_staged_kernel does the same with one voxel per thread;
+// (batch_pairs_kernel); batch_staged_kernel does the same with one voxel per thread;
 // batch_heat_kernel reads neighbours with cached global loads.
 #include <cstdint>
 
@@ -209,15 +208,13 @@ __device__ __forceinline__ float ghost_sum(const FusedArgs &a, const ClassLut &L
 constexpr int ARGS_WORDS = (int)(sizeof(FusedArgs) / 4), LUT_WORDS = (int)(sizeof(ClassLut) / 4);
 static_assert(sizeof(FusedArgs) % 4 == 0 && sizeof(ClassLut) % 4 == 0, "word copies");
 
-// K steps of every instance (GRID: persistent cooperative launch, items
-// strided over the grid, a bounded grid barrier between steps) or one step
-// with one item per block (!GRID, K == 1).  Each item streams its planes
+// K steps of every instance (persistent cooperative launch, items strided over
+// the grid, a bounded grid barrier between steps).  Each item streams its planes
 // z0-1 .. z1 through the ring, AD - 2 planes ahead of the next one needed;
 // the instance's constants and class table sit in shared memory.
 #ifndef TAM_STAGED_MINB
 #define TAM_STAGED_MINB 3
 #endif
-template <bool GRID>
 __global__ void __launch_bounds__(FX *FY, TAM_STAGED_MINB)
     batch_staged_kernel(const BatchInst *__restrict__ insts, int n, const int *__restrict__ prefix,
                         const BatchStep *__restrict__ steps, int K, BatchSync *sync, unsigned *err)
@@ -231,7 +228,7 @@ __global__ void __launch_bounds__(FX *FY, TAM_STAGED_MINB)
     unsigned char *sm = smem_raw + ((128 - ((unsigned)__cvta_generic_to_shared(smem_raw) & 127)) & 127);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * FX + tx;
     const int total = __ldg(prefix + n);
-    const int stride = GRID ? (int)gridDim.x : total;
+    const int stride = (int)gridDim.x;
     int loaded = -1;
     for (int k = 0; k < K; ++k) {
         for (int item = blockIdx.x; item < total; item += stride) {
@@ -380,7 +377,7 @@ __global__ void __launch_bounds__(FX *FY, TAM_STAGED_MINB)
             __syncthreads();  // the next item rewrites the stages and the instance's tables
             if (errbits) atomicOr(I.a.err, errbits);  // (the shared copy may already hold the next instance)
         }
-        if (GRID && k + 1 < K && !grid_barrier(sync, gridDim.x, err)) return;
+        if (k + 1 < K && !grid_barrier(sync, gridDim.x, err)) return;
     }
 }
 
@@ -467,14 +464,10 @@ __device__ __forceinline__ void issue_plane2(const Src &d, const Offs2 &o, int p
 #ifndef TAM_PAIRS_MINB
 #define TAM_PAIRS_MINB 5  // 96 registers without spills; 6 blocks spill and run 25 % slower
 #endif
-// GRID: K steps of every instance (persistent cooperative launch).  !GRID:
-// one step of one instance, one block per item; the step (`one`) and the
-// buffer pair it reads (`one_fcur`) come as parameters.
-template <bool GRID>
+// K steps of every instance (persistent cooperative launch).
 __global__ void __launch_bounds__(FX / 2 * FY, TAM_PAIRS_MINB)
     batch_pairs_kernel(const BatchInst *__restrict__ insts, int n, const int *__restrict__ prefix,
-                       const BatchStep *__restrict__ steps, int K, BatchSync *sync, unsigned *err, BatchStep one,
-                       int one_fcur)
+                       const BatchStep *__restrict__ steps, int K, BatchSync *sync, unsigned *err)
 {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(16) unsigned char s_args_raw[sizeof(FusedArgs)];
@@ -485,12 +478,12 @@ __global__ void __launch_bounds__(FX / 2 * FY, TAM_PAIRS_MINB)
     unsigned char *sm = smem_raw + ((128 - ((unsigned)__cvta_generic_to_shared(smem_raw) & 127)) & 127);
     const int tp = threadIdx.x, ty = threadIdx.y, tid = ty * (FX / 2) + tp;
     const int total = __ldg(prefix + n);
-    const int stride = GRID ? (int)gridDim.x : total;
+    const int stride = (int)gridDim.x;
     int loaded = -1;
     for (int k = 0; k < K; ++k) {
         for (int item = blockIdx.x; item < total; item += stride) {
             const Item it = item_at(insts, n, prefix, item);
-            const BatchStep st = GRID ? steps[(int64_t)k * n + it.inst] : one;
+            const BatchStep st = steps[(int64_t)k * n + it.inst];
             if (!st.active) continue;  // block-uniform
             const BatchInst &I = insts[it.inst];
             // every thread finished the previous item (its last barrier)
@@ -502,7 +495,7 @@ __global__ void __launch_bounds__(FX / 2 * FY, TAM_PAIRS_MINB)
                 loaded = it.inst;
             }
             if (tid == 0) {
-                const int fc = ((GRID ? I.fcur : one_fcur) + k) & 1;
+                const int fc = (I.fcur + k) & 1;
                 d.T = I.T[fc];
                 d.E = I.E[fc];
                 d.To = I.T[fc ^ 1];
@@ -695,7 +688,7 @@ __global__ void __launch_bounds__(FX / 2 * FY, TAM_PAIRS_MINB)
             __syncthreads();  // the next item rewrites the stages and the instance's tables
             if (errbits) atomicOr(I.a.err, errbits);
         }
-        if (GRID && k + 1 < K && !grid_barrier(sync, gridDim.x, err)) return;
+        if (k + 1 < K && !grid_barrier(sync, gridDim.x, err)) return;
     }
 }
 
@@ -836,9 +829,9 @@ cudaError_t batch_heat_blocks(int *blocks, int staged)
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = staged == 2   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_pairs_kernel<true>, FX / 2 * FY,
+        e = staged == 2   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_pairs_kernel, FX / 2 * FY,
                                                                           A_SMEM)
-            : staged == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_staged_kernel<true>, FX * FY,
+            : staged == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_staged_kernel, FX * FY,
                                                                           A_SMEM)
                           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_heat_kernel, FX * FY, 0);
     if (e != cudaSuccess) return e;
@@ -852,30 +845,16 @@ cudaError_t launch_batch_heat(const BatchInst *insts, int n, const int *prefix, 
     if (n <= 0 || K <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(sync, 0, sizeof(BatchSync), s);
     if (e != cudaSuccess) return e;
-    BatchStep one{};
-    int one_fcur = 0;
     void *args[] = {(void *)&insts, (void *)&n, (void *)&prefix, (void *)&steps, (void *)&K, (void *)&sync,
                     (void *)&err};
-    void *args2[] = {(void *)&insts, (void *)&n,    (void *)&prefix, (void *)&steps,   (void *)&K,
-                     (void *)&sync,  (void *)&err,  (void *)&one,    (void *)&one_fcur};
     count_launch();
     if (staged == 2)
-        return cudaLaunchCooperativeKernel((const void *)batch_pairs_kernel<true>, dim3(blocks), dim3(FX / 2, FY),
-                                           args2, A_SMEM, s);
+        return cudaLaunchCooperativeKernel((const void *)batch_pairs_kernel, dim3(blocks), dim3(FX / 2, FY),
+                                           args, A_SMEM, s);
     if (staged == 1)
-        return cudaLaunchCooperativeKernel((const void *)batch_staged_kernel<true>, dim3(blocks), dim3(FX, FY), args,
+        return cudaLaunchCooperativeKernel((const void *)batch_staged_kernel, dim3(blocks), dim3(FX, FY), args,
                                            A_SMEM, s);
     return cudaLaunchCooperativeKernel((const void *)batch_heat_kernel, dim3(blocks), dim3(FX, FY), args, 0, s);
-}
-
-cudaError_t launch_staged_step(const BatchInst *inst, const int *prefix, int items, const BatchStep &step, int fcur,
-                               cudaStream_t s)
-{
-    if (items <= 0) return cudaSuccess;
-    count_launch();
-    batch_pairs_kernel<false><<<items, dim3(FX / 2, FY), A_SMEM, s>>>(inst, 1, prefix, nullptr, 1, nullptr, nullptr,
-                                                                       step, fcur);
-    return cudaGetLastError();
 }
 
 }  // namespace tam

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "f32x2.cuh"
 #include "heat_common.cuh"
 #include "slab_common.cuh"
 
@@ -42,31 +43,6 @@ namespace {
 constexpr int QTPB = 128;  // threads per block (256: 1-3 % slower; 64: 10 %)
 constexpr int QZMAX = 8;   // planes per block at most (the list holds every voxel of a block)
 
-// two FP32 operations in one instruction, each rounded as its scalar form
-#define TAM_F32X2(name, op)                                                                                  \
-    __device__ __forceinline__ float2 name(float2 a, float2 b)                                               \
-    {                                                                                                        \
-        float2 r;                                                                                            \
-        asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t" op                     \
-            ".rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"                                                \
-            : "=f"(r.x), "=f"(r.y)                                                                           \
-            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                       \
-        return r;                                                                                            \
-    }
-TAM_F32X2(add2, "add")
-TAM_F32X2(sub2, "sub")
-TAM_F32X2(mul2, "mul")
-#undef TAM_F32X2
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
-{
-    float2 r;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-        "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return r;
-}
-__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 lo2(const float4 &v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(const float4 &v) { return make_float2(v.z, v.w); }
 // (plain loads: the step before may still be writing when this kernel starts,
@@ -398,11 +374,11 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
         for (int n = threadIdx.x; n < nf; n += QTPB) {
             const int l = s_faces[n >> 2];
             const int vp = 4 * (int)(q0 + l % QTPB) + (n & 3), z = z0 + l / QTPB, v = vp + pl * z, yy = vp / nx, xx = vp - yy * nx;
-            const int cp = C.cpitch, ci = xx + cp * (yy + ny * z);
+            const int64_t cp = C.cpitch, ci = xx + cp * (yy + (int64_t)ny * z);
             const int k = C.cls[ci] & (MAX_MAT - 1);
             const float tc = T[v], e0 = E[v], kk = L.k[k];
             const float *frow = s_fa + k * MAX_MAT;
-            auto face = [&](bool in, int f, int dv, int dc, float &t, float &e) -> float {
+            auto face = [&](bool in, int f, int dv, int64_t dc, float &t, float &e) -> float {
                 if (in) {
                     t = T[v + dv];
                     e = E[v + dv];
@@ -472,7 +448,7 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
 
 bool quad_step_supported(int nx, int ny, int nz)
 {
-    return nx > 0 && nx % 4 == 0 && (int64_t)nx * ny * nz < ((int64_t)1 << 31) - 64;
+    return nx > 0 && nx % 4 == 0 && nz <= QZMAX * 65535 && (int64_t)nx * ny * nz < ((int64_t)1 << 31) - 64;
 }
 
 static int64_t tiles_of(int nx, int ny, int nz) { return (int64_t)((nx + TW - 1) / TW) * ((ny + TR - 1) / TR) * nz; }

@@ -143,11 +143,9 @@ struct tam_ctx {
     int batch_streams = 0;           // 1: batched steps as each instance's own steps on its stream, overlapped
     int batch_transport = 1;         // batched loops: the instances' uniform-medium passes in one launch
     int batch_zchunk = 0;            // batched steps: z planes per work item (0: heat.zchunk, else the default)
-    // staged class-table step of this context alone (rows not aligned for TMA)
-    tam::BatchInst *d_sinst = nullptr;
-    int *d_sprefix = nullptr;
-    tam::BatchInst h_sinst{};
-    int s_items = 0;
+    // line form of the class-table step (rows of any width): its face table
+    float *d_ltab = nullptr;
+    bool ltab_ok = false;
     tam::FusedCls *fcls = nullptr;
     // quad form of the class-table step: the quads' table on a heterogeneous
     // grid, made when a heat call finds it out of date
@@ -475,7 +473,7 @@ int set_thermal_classes(tam_ctx *ctx, int u)
     ctx->cls64_ok = false;
     if (ctx->d_cls)
         CK(tam::launch_cls_from_mat(ctx->d_mat, nm, ctx->d_cls, ctx->nx, ctx->ny, ctx->nz, ctx->cls_pitch, ctx->stream));
-    ctx->qs_ok = false;
+    ctx->qs_ok = ctx->ltab_ok = false;
     return TAM_OK;
 }
 
@@ -912,10 +910,9 @@ int ref_damage_props(tam_ctx *ctx, double ablate_temp)
 }
 
 // --------------------------------------------------------- heat (config) --
-// Default z planes per work item of the staged step: long columns for the
-// batched launch (fewer halo planes; the batch's items fill the device) and
-// shorter ones for one context alone (enough items for every SM).
-constexpr int BATCH_ZCHUNK = 32, SINGLE_ZCHUNK = 8, BATCH_SLAB_ZCHUNK = 32;
+// Default z planes per work item of the batched step: long columns (fewer halo
+// planes; the batch's items fill the device).
+constexpr int BATCH_ZCHUNK = 32, BATCH_SLAB_ZCHUNK = 32;
 
 // The batched-step description of one context; returns its work items.
 // z planes per item: zforce if positive, else the context's heat.zchunk if
@@ -939,29 +936,13 @@ int batch_inst(tam_ctx *c, tam::BatchInst &I, int zdefault, int zforce = 0)
     return I.tiles_x * I.tiles_y * ((c->nz + I.zchunk - 1) / I.zchunk);
 }
 
-// Device description of this context for the staged class-table step (its
-// rows are not 16-byte aligned for TMA, or TMA is off), rebuilt before each
-// run of steps and copied only when it changed (classes, constants, tuning).
-// The per-step source, time and buffer pair travel as kernel parameters.
-int staged_setup(tam_ctx *ctx)
+// The line form's face table.
+int line_table(tam_ctx *ctx)
 {
-    if (!ctx->d_sinst) {
-        RC(dalloc_t(ctx, &ctx->d_sinst, 1));
-        RC(dalloc_t(ctx, &ctx->d_sprefix, 2));
-    }
-    tam::BatchInst I{};
-    const int items = batch_inst(ctx, I, SINGLE_ZCHUNK);
-    I.a.P = 0.0;
-    I.a.t_new = 0.0;
-    I.fcur = 0;
-    if (items != ctx->s_items || std::memcmp(&I, &ctx->h_sinst, sizeof I) != 0) {
-        // pageable sources: the copies take the bytes before they return
-        ctx->h_sinst = I;
-        ctx->s_items = items;
-        const int pre[2] = {0, items};
-        CK(cudaMemcpyAsync(ctx->d_sinst, &ctx->h_sinst, sizeof I, cudaMemcpyHostToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(ctx->d_sprefix, pre, sizeof pre, cudaMemcpyHostToDevice, ctx->stream));
-    }
+    if (ctx->ltab_ok) return TAM_OK;
+    if (!ctx->d_ltab) RC(dalloc_t(ctx, &ctx->d_ltab, tam::LINE_TABLE));
+    CK(tam::launch_line_table(ctx->clut, ctx->d_ltab, ctx->stream));
+    ctx->ltab_ok = true;
     return TAM_OK;
 }
 
@@ -999,13 +980,13 @@ int cls64_setup(tam_ctx *ctx)
 }
 
 // Forms of the config-mode heat step, by what the context's state allows.
-enum HeatForm { HF_CLS = 0, HF_STAGED, HF_TMA, HF_CPASYNC, HF_QUAD, HF_CLS64 };
+enum HeatForm { HF_CLS = 0, HF_LINE, HF_TMA, HF_CPASYNC, HF_QUAD, HF_CLS64 };
 
 HeatForm heat_form(const tam_ctx *ctx)
 {
     if (ctx->quad && ctx->use_slab && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class) return HF_QUAD;
     if (ctx->fcls && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class) return HF_CLS;
-    if (!ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && ctx->d_cls) return HF_STAGED;
+    if (!ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && ctx->d_cls && tam::line_step_supported(ctx->nx, ctx->ny, ctx->nz)) return HF_LINE;
     if (ctx->tma && ctx->use_tma) return HF_TMA;
     if (ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && (ctx->cls_uniform >= 0 || ctx->cls64_ok)) return HF_CLS64;
     return HF_CPASYNC;
@@ -1021,14 +1002,7 @@ int launch_heat(tam_ctx *ctx, tam::FusedArgs &a, HeatForm form, int which, cudaS
     switch (form) {
     case HF_QUAD: CK(tam::launch_quad_step(a, ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->d_qs, s)); break;
     case HF_CLS: CK(tam::launch_fused_cls(a, ctx->fcls, which, ctx->clut, ctx->cls_rows, s)); break;
-    case HF_STAGED: {
-        tam::BatchStep st{};
-        st.t_new = a.t_new;
-        st.pdt = (float)(a.P * ctx->cdt);
-        st.active = 1;
-        CK(tam::launch_staged_step(ctx->d_sinst, ctx->d_sprefix, ctx->s_items, st, which, s));
-        break;
-    }
+    case HF_LINE: CK(tam::launch_line_step(a, ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->d_ltab, s)); break;
     case HF_TMA: CK(tam::launch_fused_tma(a, ctx->tma, which, s)); break;
     case HF_CLS64: CK(tam::launch_cls64_step(a, ctx->clut64, ctx->d_cls64, s)); break;
     default: CK(tam::launch_fused_step(a, ctx->fp64, s)); break;
@@ -1119,12 +1093,12 @@ int cfg_heat(tam_ctx *ctx, int32_t nsteps, int32_t *done = nullptr, bool stop_on
     if (nsteps > 0) RC(cls64_setup(ctx));
     if (heat_form(ctx) == HF_QUAD && nsteps > 0) RC(quad_classes(ctx));
     const HeatForm form = heat_form(ctx);
-    if (form == HF_STAGED && nsteps > 0) RC(staged_setup(ctx));
+    if (form == HF_LINE && nsteps > 0) RC(line_table(ctx));
     if (form == HF_TMA && ctx->coeff_dirty && nsteps > 0) {
         CK(tam::launch_face_coeffs(a, ctx->d_ax, ctx->d_ay, ctx->d_az, ctx->d_irc, ctx->stream));
         ctx->coeff_dirty = false;
     }
-    const bool graphs = ctx->use_graph && form != HF_STAGED && nsteps >= GRAPH_STEPS;
+    const bool graphs = ctx->use_graph && nsteps >= GRAPH_STEPS;
     std::vector<unsigned char> key;
     if (graphs) key = graph_key(ctx, a, form);
     // re-trace check after a step: every `check` heat steps, counted across
@@ -2939,7 +2913,7 @@ int tam_set_tuning(tam_ctx *ctx, const char *key, int64_t value)
     } else if (k == "heat.zchunk") {
         if (value < 0 || value > ctx->nz) return fail(ctx, TAM_E_INVALID, "heat.zchunk must be in 0..nz");
         ctx->zchunk = (int)value;
-        ctx->qs_ok = false;
+        ctx->qs_ok = ctx->ltab_ok = false;
     } else {
         return fail(ctx, TAM_E_INVALID, "unknown tuning key " + k);
     }
@@ -3130,7 +3104,7 @@ int tam_load_state(tam_ctx *ctx, const char *path)
         if (!f) return fail(ctx, TAM_E_PARSE, "state file truncated");
         CK(cudaMemcpy(b.first, host.data(), n, cudaMemcpyHostToDevice));
     }
-    ctx->qs_ok = false;  // follows the class grid just loaded
+    ctx->qs_ok = ctx->ltab_ok = false;  // follows the class grid just loaded
     set_scalars(ctx, S);
     std::memcpy(ctx->tally, tally, sizeof tally);
     ctx->tally_stale = false;
@@ -3244,7 +3218,7 @@ int tam_autotune(tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, 
         ctx->use_slab = slab0;
         (void)cudaGetLastError();
         (void)snap_restore(ctx, S);
-        ctx->qs_ok = false;
+        ctx->qs_ok = ctx->ltab_ok = false;
         return code;
     };
     auto timed = [&](int ev0, int ev1) -> int {
@@ -3278,15 +3252,14 @@ int tam_autotune(tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, 
         float best_ms = 1e30f;
         const bool cls = ctx->fcls && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class;
         const bool slab = ctx->quad && ctx->use_tma && ctx->use_cls && ctx->thermal_by_class;
-        const bool staged = !cls && !slab && !ctx->fp64 && ctx->use_cls && ctx->thermal_by_class && ctx->d_cls;
-        const std::vector<int> zcs = staged ? std::vector<int>{4, 8, 16, 32} : std::vector<int>{2, 3, 4, 5, 8, 16};
+        const std::vector<int> zcs{2, 3, 4, 5, 8, 16};
         for (int form : {2, 0, 1}) {  // 2: quad form; 0 / 1: class-table voxel pairs / rows
             if (form == 2 && !slab) continue;
             if (form == 0 && !cls) continue;
             for (int zc : zcs) {
                 if (zc > ctx->nz) continue;
                 ctx->zchunk = zc;
-                ctx->qs_ok = false;
+                ctx->qs_ok = ctx->ltab_ok = false;
                 ctx->use_slab = form == 2;
                 if (form != 2) ctx->cls_rows = form;
                 if ((r = cfg_heat(ctx, steps)) != TAM_OK || (r = timed(2, 3)) != TAM_OK ||
@@ -3301,7 +3274,7 @@ int tam_autotune(tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, 
             }
         }
         ctx->zchunk = best_z;
-        ctx->qs_ok = false;
+        ctx->qs_ok = ctx->ltab_ok = false;
         ctx->cls_rows = best_r;
         ctx->use_slab = best_s;
     }

@@ -353,6 +353,13 @@ bool quad_step_supported(int nx, int ny, int nz);
 int64_t quad_class_bytes(int nx, int ny, int nz);
 cudaError_t launch_quad_classes(const ClassLut &L, const uint8_t *cls, int pitch, int nx, int ny, int nz, int zchunk,
                                 uint8_t *qs, cudaStream_t s);
+// Line form (heat_line.cu): rows of any width, fewer than 2^31 voxels.  tab:
+// LINE_TABLE floats, the face table of a heterogeneous grid.
+constexpr int LINE_TABLE = MAX_MAT * MAX_MAT;
+bool line_step_supported(int nx, int ny, int nz);
+cudaError_t launch_line_table(const ClassLut &L, float *tab, cudaStream_t s);
+cudaError_t launch_line_step(const FusedArgs &a, const ClassLut &L, const uint8_t *cls, int cpitch, const float *tab,
+                             cudaStream_t s);
 // One step, as a programmatic dependent of the launch before it.
 cudaError_t launch_quad_step(const FusedArgs &a, const ClassLut &L, const uint8_t *cls, int cpitch, const uint8_t *qs,
                              cudaStream_t s);
@@ -403,11 +410,6 @@ constexpr int BATCH_STEP_ZMAX = 128;
 cudaError_t launch_batch_slab_steps(const BatchInst *insts, int n, const int *prefix, int items, int zmax,
                                     const int *vox0, const BatchStep *steps, int K, unsigned *rare,
                                     unsigned *rare_cnt, unsigned *err, bool uniform, int sm_count, cudaStream_t s);
-// One step of one instance (inst: device copy of its BatchInst) by the staged
-// voxel-pair kernel, one block per work item (prefix = {0, items}); any row
-// pitch.  fcur selects the buffer pair read by the step.
-cudaError_t launch_staged_step(const BatchInst *inst, const int *prefix, int items, const BatchStep &step, int fcur,
-                               cudaStream_t s);
 
 // The isolation rule of src/3dFD.f90:347-349 on the config-mode material
 // grid: a voxel that is not air (id != 0) and whose six neighbours are air
