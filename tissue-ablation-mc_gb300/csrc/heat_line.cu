@@ -94,8 +94,7 @@ __global__ void __launch_bounds__(LTPB, 8)
     const unsigned q0 = blockIdx.x * LV;
     // runs of planes from the top face down: the beam enters there, so the
     // blocks with the longest lists start first
-    const int nzc = (nz + zchunk - 1) / zchunk;
-    const int z0 = (nzc - 1 - (int)blockIdx.y) * zchunk, z1 = min(nz, z0 + zchunk);
+    const int z0 = (int)(gridDim.y - 1 - blockIdx.y) * zchunk, z1 = min(nz, z0 + zchunk);
     const float *T = (const float *)a.T_in, *E = a.Tc_in, *J = (const float *)a.J;
     float *To = (float *)a.T_out, *Eo = a.Tc_out;
     const int uc = L.uniform >= 0 ? L.uniform : 0;
