@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/tam.h"
+#include "prefault.h"
 #include "tam_kernels.h"
 #include "tam_util.h"
 
@@ -1937,6 +1938,7 @@ int tam_mc_pass(tam_ctx *ctx, int64_t nphotons, uint64_t seed, uint32_t stream, 
     if (!ctx) return fail(nullptr, TAM_E_INVALID, "null context");
     if (nphotons < 0) return fail(ctx, TAM_E_INVALID, "nphotons must be >= 0");
     CK(cudaSetDevice(ctx->device));
+    tam::Prefault pages(jmean_out, jmean_out ? (size_t)ctx->ni * 8 : 0);
     RC(mc_pass(ctx, nphotons, seed, stream));
     if (ctx->config) {
         unsigned long long nab = 0;
@@ -1944,6 +1946,7 @@ int tam_mc_pass(tam_ctx *ctx, int64_t nphotons, uint64_t seed, uint32_t stream, 
         ctx->nabl_at_trace = (long long)nab;
         ctx->need_trace = false;
     }
+    pages.end();
     if (jmean_out) return tam_download(ctx, TAM_F_JMEAN_GLOBAL, jmean_out, ctx->ni * 8);
     return TAM_OK;
 }
@@ -1953,8 +1956,10 @@ int tam_heat_steps(tam_ctx *ctx, int32_t nsteps, double *temp_out)
     if (!ctx) return fail(nullptr, TAM_E_INVALID, "null context");
     if (nsteps < 0) return fail(ctx, TAM_E_INVALID, "nsteps must be >= 0");
     CK(cudaSetDevice(ctx->device));
+    tam::Prefault pages(temp_out, temp_out ? (size_t)ctx->nh * 8 : 0);
     RC(ctx->config ? cfg_heat(ctx, nsteps) : ref_heat(ctx, nsteps));
     RC(finish(ctx, "tam_heat_steps"));
+    pages.end();
     if (temp_out) return tam_download(ctx, TAM_F_TEMP, temp_out, ctx->nh * 8);
     return TAM_OK;
 }
