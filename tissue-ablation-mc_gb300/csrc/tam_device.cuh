@@ -80,7 +80,11 @@ __host__ __device__ inline void philox_round_keys(uint64_t seed, uint32_t *rk)
 template <typename Real> struct Uniform;
 // FP64: u = (x + 0.5) 2^-32, exact in (0,1).
 template <> struct Uniform<double> {
-    __device__ __forceinline__ static double from(uint32_t x) { return ((double)x + 0.5) * 0x1p-32; }
+    // (x from the bits of 2^52 + x: an integer-to-double conversion runs on the FP64 pipe too)
+    __device__ __forceinline__ static double from(uint32_t x)
+    {
+        return __fma_rn(__hiloint2double(0x43300000, (int)x) - 0x1p52, 0x1p-32, 0x1p-33);
+    }
 };
 // FP32: u = ((x >> 9) + 0.5) 2^-23: k + 0.5 is exact in FP32 for k < 2^23, so
 // u lies on a 2^-23 grid strictly inside (0,1), the largest value 1 - 2^-24.

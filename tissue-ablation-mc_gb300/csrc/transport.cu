@@ -137,6 +137,9 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     __shared__ double s_tal[5];  // specular, reflected, transmitted, side, roulette net
     __shared__ unsigned long long s_cnt[2];  // voxel steps, scatters
     __shared__ unsigned s_err;
+    constexpr bool SCAT64 = sizeof(Real) == 8 && MED != MED_RHOKAP;  // the reference medium only absorbs
+    __shared__ double2 s_turn[SCAT64 ? TURN + 1 : 1];
+    if constexpr (SCAT64) turn_table(s_turn);
     if (threadIdx.x < 5) s_tal[threadIdx.x] = 0.0;
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
     if (threadIdx.x == 0) s_err = 0u;
@@ -176,8 +179,8 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     bool exhausted = false;
     int ix = 0, iy = 0, iz = 0, mid = 0, sgx = 1, sgy = 1, sgz = 1;
     auto cell = [&]() { return ix + NX * (iy + NY * iz); };
-    Real fx = 0, fy = 0, fz = 0, nx = 0, ny = 0, nz = 0, sint = 0, phi = 0;
-    Real cpv = 1, spv = 0;  // FP32 path: (cos phi, sin phi) in place of phi
+    Real fx = 0, fy = 0, fz = 0, nx = 0, ny = 0, nz = 0, sint = 0;
+    Real cpv = 1, spv = 0;  // (cos phi, sin phi)
     Real tdx = 0, tdy = 0, tdz = 0, tmx = 0, tmy = 0, tmz = 0, t = 0;
     Real w = 0, tau = 0, dep = 0, mut = 0, mua = 0;
     uint32_t ev = 0, plo = 0, phi32 = 0, nsteps = 0;
@@ -226,17 +229,16 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     Real st, ct, sp, cp;
                     M<Real>::sincos(u1 * TWOPI, &st, &ct);
                     const Real X = rad * ct + K.xmax, Y = rad * st + K.ymax;
-                    phi = TWOPI * u2;
                     if constexpr (MED == MED_RHOKAP) {
                         // reference medium: a pure absorber (any interaction
                         // ends the packet) launched straight down, so the
                         // azimuth only enters nx = ny = sint * (cos, sin) phi
-                        // = +-0, which the walk treats alike; its sincos (an
-                        // FP64 one in the parity form) is skipped
+                        // = +-0, which the walk treats alike; its sincos is skipped
                         cp = (Real)1;
                         sp = (Real)0;
                     } else {
-                        M<Real>::sincos(phi, &sp, &cp);
+                        if constexpr (SCAT64) turn(s_turn, r.z, sp, cp);
+                        else M<Real>::sincos(TWOPI * u2, &sp, &cp);
                     }
                     cpv = cp;
                     spv = sp;
@@ -437,11 +439,12 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     nx = -nx;
                     sgx = -sgx;
                     tmx = t + tdx;
-                    if constexpr (sizeof(Real) == 4) {
-                        cpv = -cpv;  // phi -> PI - phi
+                    if constexpr (SCAT64) {
+                        const Azimuth p = mirror_x(Azimuth{cpv, spv});
+                        cpv = p.c;
+                        spv = p.s;
                     } else {
-                        phi = (Real)PI_R - phi;
-                        if (phi < (Real)0) phi += TWOPI;
+                        cpv = -cpv;  // phi -> PI - phi
                     }
                 } else if (cy) {
                     iy -= sgy;
@@ -451,10 +454,12 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     ny = -ny;
                     sgy = -sgy;
                     tmy = t + tdy;
-                    if constexpr (sizeof(Real) == 4) {
-                        spv = -spv;  // phi -> TWOPI - phi
+                    if constexpr (SCAT64) {
+                        const Azimuth p = mirrored(Azimuth{cpv, spv}, COS_2PI, SIN_2PI);
+                        cpv = p.c;
+                        spv = p.s;
                     } else {
-                        phi = TWOPI - phi;
+                        spv = -spv;  // phi -> TWOPI - phi
                     }
                 } else {
                     iz -= sgz;
@@ -511,27 +516,31 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                 } else {
                     interact();
                     bool die = !(w > (Real)0);
-                    if (!die) {
-                        const U4 r = philox4x32_10_rk(ev++, plo, phi32, strm, a.rk);
-                        cScat += 1;
-                        fx = axis_pos(nx, fx, hx, tmx, t);
-                        fy = axis_pos(ny, fy, hy, tmy, t);
-                        fz = axis_pos(nz, fz, hz, tmz, t);
-                        Real cost = nz, cp, sp;
-                        if (stokes<Real>(lut[mid].g, lut[mid].g2, Uniform<Real>::from(r.x), Uniform<Real>::from(r.y), cost,
-                                         sint, phi, cp, sp)) {
-                            nx = sint * cp;
-                            ny = sint * sp;
-                            nz = cost;
-                        }
-                        if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
-                            atomicOr(&s_err, (unsigned)DEVERR_NAN);
-                            die = true;
-                        } else {
-                            setup();
-                            t = (Real)0;
-                            die = a.roulette && w < wmin && !roulette(r.z);
-                            tau = M<Real>::neglog(Uniform<Real>::from(r.w));
+                    if constexpr (SCAT64) {
+                        if (!die) {
+                            const U4 r = philox4x32_10_rk(ev++, plo, phi32, strm, a.rk);
+                            cScat += 1;
+                            fx = axis_pos(nx, fx, hx, tmx, t);
+                            fy = axis_pos(ny, fy, hy, tmy, t);
+                            fz = axis_pos(nz, fz, hz, tmz, t);
+                            double cost = nz;
+                            Azimuth p{cpv, spv};
+                            if (stokes(s_turn, lut[mid].g, lut[mid].g2, r.x, r.y, cost, sint, p)) {
+                                cpv = p.c;
+                                spv = p.s;
+                                nx = sint * cpv;
+                                ny = sint * spv;
+                                nz = cost;
+                            }
+                            if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
+                                atomicOr(&s_err, (unsigned)DEVERR_NAN);
+                                die = true;
+                            } else {
+                                setup();
+                                t = (Real)0;
+                                die = a.roulette && w < wmin && !roulette(r.z);
+                                tau = M<Real>::neglog(Uniform<Real>::from(r.w));
+                            }
                         }
                     }
                     if (die) end();

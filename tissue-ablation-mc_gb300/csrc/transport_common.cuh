@@ -12,58 +12,108 @@
 namespace tam {
 namespace {
 
-// HG deflection with the arithmetic of src/stokes.f90:6-153 (PI/TWOPI are
-// the truncated constants of src/constants.f90:13).  Leaves the direction
-// unchanged when the sampled cosine is exactly +-1 (the `goto 100`).
-template <typename Real>
-__device__ __forceinline__ bool stokes(Real hgg, Real g2, Real u0, Real u1, Real &cost, Real &sint, Real &phi,
-                                       Real &cosp, Real &sinp)
+// (sin, cos) of TWOPI u, u = (x + 1/2) 2^-32 (TWOPI: the truncated constant of
+// src/constants.f90:13), from a table of 256 steps of the turn and the Taylor terms
+// of the rest, at most 0.0123: next terms 8e-18 and 1e-20.  16 FP64 operations against
+// some 45 of the library's, and the angle itself is never rounded.
+constexpr int TURN = 256;
+__device__ __forceinline__ void turn_table(double2 *tab)
 {
-    const Real PI = (Real)PI_R, TWOPI = (Real)TWOPI_R;
-    const Real one = (Real)1;
-    if (hgg == (Real)0) {
-        cost = (Real)2 * u0 - one;
-        Real s2 = one - cost * cost;
-        sint = s2 <= (Real)0 ? (Real)0 : M<Real>::sqrt(s2);
-        phi = TWOPI * u1;
-        M<Real>::sincos(phi, &sinp, &cosp);
+    for (int i = threadIdx.x; i <= TURN; i += blockDim.x) ::sincos(TWOPI_R * (i * (1.0 / TURN)), &tab[i].x, &tab[i].y);
+}
+__device__ __forceinline__ void turn(const double2 *tab, uint32_t x, double &sn, double &cs)
+{
+    const uint32_t i = ((x >> 23) + 1u) >> 1;
+    const int r = (int)(x - (i << 24));
+    const double k = TWOPI_R * 0x1p-32;
+    const double b = __fma_rn(__hiloint2double(0x43380000 + (r >> 31), r) - 0x1.8p52, k, 0.5 * k), b2 = b * b;
+    const double sb = __fma_rn(b * b2, __fma_rn(b2, 1.0 / 120, -1.0 / 6), b);
+    const double cm = b2 * __fma_rn(b2, __fma_rn(b2, -1.0 / 720, 1.0 / 24), -0.5);
+    const double2 t = tab[i];
+    sn = t.x + __fma_rn(t.x, cm, t.y * sb);
+    cs = t.y + __fma_rn(t.y, cm, -(t.x * sb));
+}
+// An azimuth in [0, TWOPI] as (cos, sin); cos and sin of the truncated constants.
+struct Azimuth {
+    double c, s;
+};
+constexpr double COS_PI = -0x1.ffffffffff87cp-1, SIN_PI = 0x1.5ee4b2791a46fp-21;
+constexpr double COS_2PI = 0x1.ffffffffffe57p-1, SIN_2PI = -0x1.49d4e1c46983ep-22;
+// phi -> a - phi, phi -> phi + a, phi -> phi - a for an angle a given as (ca, sa)
+__device__ __forceinline__ Azimuth mirrored(Azimuth p, double ca, double sa) { return {ca * p.c + sa * p.s, sa * p.c - ca * p.s}; }
+__device__ __forceinline__ Azimuth turned(Azimuth p, double ca, double sa) { return {p.c * ca - p.s * sa, p.s * ca + p.c * sa}; }
+// phi -> PI - phi, plus TWOPI below 0
+__device__ __forceinline__ Azimuth mirror_x(Azimuth p)
+{
+    const Azimuth q = mirrored(p, COS_PI, SIN_PI);
+    return p.s < 0.0 || (p.c < 0.0 && p.s < SIN_PI) ? turned(q, COS_2PI, SIN_2PI) : q;
+}
+
+// HG deflection of src/stokes.f90:6-153 (PI/TWOPI are the truncated constants of
+// src/constants.f90:13).  Leaves the direction unchanged when the sampled cosine is
+// exactly +-1 (the `goto 100`).  The azimuth is carried as (cos, sin) and turned by
+// the deflection angle, whose cosine is at hand: no acos, and no sincos of the sum.
+// The reference wraps phi by the truncated TWOPI, a turn of 3e-7: wrapped here at the
+// same angles.
+//
+// The FP64 pipe bounds the walk (82 % busy), and a scatter took some 310 of its
+// operations; without the acos and that sincos 255: 1e6 packets through a 100^3
+// cube 181 -> 165 ms.  The cosine of the deflection keeps its operations one by one:
+// near +-1 the angle multiplies its last bit by 1e8.
+__device__ __forceinline__ bool stokes(const double2 *tab, double hgg, double g2, uint32_t d0, uint32_t d1, double &cost,
+                                       double &sint, Azimuth &phi)
+{
+    const double u0 = Uniform<double>::from(d0);
+    if (hgg == 0.0) {
+        cost = 2.0 * u0 - 1.0;
+        const double s2 = 1.0 - cost * cost;
+        sint = s2 <= 0.0 ? 0.0 : ::sqrt(s2);
+        turn(tab, d1, phi.s, phi.c);
         return true;
     }
-    const Real costp = cost, sintp = sint, phip = phi;
-    const Real t = M<Real>::div(one - g2, one - hgg + (Real)2 * hgg * u0);
-    Real bmu = M<Real>::div((one + g2) - t * t, (Real)2 * hgg);
-    Real cosb2 = bmu * bmu;
-    if (M<Real>::abs(bmu) > one) {
-        bmu = bmu > one ? one : -one;
-        cosb2 = one;
+    const double costp = cost, sintp = sint;
+    const double t = (1.0 - g2) / (1.0 - hgg + 2.0 * hgg * u0);
+    double bmu = ((1.0 + g2) - t * t) / (2.0 * hgg);
+    double cosb2 = bmu * bmu;
+    if (fabs(bmu) > 1.0) {
+        bmu = bmu > 1.0 ? 1.0 : -1.0;
+        cosb2 = 1.0;
     }
-    if (bmu == one || bmu == -one) return false;  // direction unchanged
-    const Real sinbt = M<Real>::sqrt(one - cosb2);
-    const Real ri1 = TWOPI * u1;
-    const bool upper = ri1 > PI;
-    const Real ang = upper ? TWOPI - ri1 : ri1;
-    Real sa, ca;
-    M<Real>::sincos(ang, &sa, &ca);
-    Real cosi2 = (Real)0, sini2;
+    if (bmu == 1.0 || bmu == -1.0) return false;  // direction unchanged
+    const double sinbt = ::sqrt(1.0 - cosb2);
+    const double ri1 = TWOPI_R * Uniform<double>::from(d1);
+    const bool upper = ri1 > PI_R;
+    const double ang = upper ? TWOPI_R - ri1 : ri1;
+    double sa, ca;
+    ::sincos(ang, &sa, &ca);
+    double cosi2 = 0.0, sini2;
     cost = costp * bmu + sintp * sinbt * ca;
-    if (M<Real>::abs(cost) < one) {
-        sint = M<Real>::abs(M<Real>::sqrt(one - cost * cost));
-        sini2 = M<Real>::div(sa * sintp, sint);
-        const Real bott = sint * sinbt;
-        cosi2 = M<Real>::div(costp, bott) - M<Real>::div(cost * bmu, bott);
+    if (fabs(cost) < 1.0) {
+        sint = fabs(::sqrt(1.0 - cost * cost));
+        sini2 = sa * sintp / sint;
+        const double bott = sint * sinbt;
+        cosi2 = costp / bott - cost * bmu / bott;
     } else {
-        sint = (Real)0;
-        sini2 = (Real)0;
-        if (cost >= one) cosi2 = -one;
-        if (cost <= -one) cosi2 = one;
+        sint = 0.0;
+        sini2 = 0.0;
+        if (cost >= 1.0) cosi2 = -1.0;
+        if (cost <= -1.0) cosi2 = 1.0;
     }
-    Real cosdph = -cosi2 * ca + sini2 * sa * bmu;
-    if (M<Real>::abs(cosdph) > one) cosdph = cosdph > one ? one : -one;
-    const Real dph = M<Real>::acos(cosdph);
-    phi = upper ? phip + dph : phip - dph;
-    if (phi > TWOPI) phi = phi - TWOPI;
-    if (phi < (Real)0) phi = phi + TWOPI;
-    M<Real>::sincos(phi, &sinp, &cosp);
+    double cd = -cosi2 * ca + sini2 * sa * bmu;
+    if (fabs(cd) > 1.0) cd = cd > 1.0 ? 1.0 : -1.0;
+    double sd = ::sqrt((1.0 - cd) * (1.0 + cd));
+    sd = upper ? sd : -sd;
+    const Azimuth p = phi;
+    phi = turned(p, cd, sd);
+    // above TWOPI: minus TWOPI; below 0: plus TWOPI (a turn by up to PI from [0, TWOPI])
+    bool over = phi.s > SIN_2PI && phi.c > 0.0 && (p.s < 0.0 || phi.s < 0.0);
+    over = upper && (over || (p.s < 0.0 && phi.s >= 0.0));
+    if (over) phi = turned(phi, COS_2PI, -SIN_2PI);
+    else if (!upper && p.s >= 0.0 && phi.s < 0.0) phi = turned(phi, COS_2PI, SIN_2PI);
+    // back to length 1 (one Newton step)
+    const double k = 1.5 - 0.5 * (phi.c * phi.c + phi.s * phi.s);
+    phi.c *= k;
+    phi.s *= k;
     return true;
 }
 
