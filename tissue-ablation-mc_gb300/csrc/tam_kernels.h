@@ -53,6 +53,8 @@ template <typename Real> struct TrConst {
     Real xmax, ymax;
     Real wmin, rm, inv_rm;            // roulette threshold, survival factor and its inverse
     Real namb, rhokap_n, src_r;       // ambient and rhokap-medium refractive indices, source radius
+    Real cells_x, cells_y;            // cells per length at launch, nx / (2 xmax)
+    Real rhokap_spec;                 // normal reflectance of the rhokap medium
 };
 
 // One material's optics in the transport's precision.

@@ -138,8 +138,6 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     __shared__ unsigned long long s_cnt[2];  // voxel steps, scatters
     __shared__ unsigned s_err;
     constexpr bool SCAT64 = sizeof(Real) == 8 && MED != MED_RHOKAP;  // the reference medium only absorbs
-    __shared__ double2 s_turn[SCAT64 ? TURN + 1 : 1];
-    if constexpr (SCAT64) turn_table(s_turn);
     if (threadIdx.x < 5) s_tal[threadIdx.x] = 0.0;
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
     if (threadIdx.x == 0) s_err = 0u;
@@ -185,6 +183,11 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     Real w = 0, tau = 0, dep = 0, mut = 0, mua = 0;
     uint32_t ev = 0, plo = 0, phi32 = 0, nsteps = 0;
     uint32_t cScat = 0;
+    // The specular tally: FP64 additions to one shared word go lane by lane, 32 of them
+    // whenever a warp launches together, and a packet of the reference medium does
+    // little else.  (FP32: the sum costs more than the contention, 0.8 us per pass.)
+    constexpr bool SPEC_REG = sizeof(Real) == 8;
+    double spec = 0.0;
     uint64_t cSteps = 0;  // voxel steps of this thread's finished packets (reduced once at the end)
     auto props = [&]() {
         if constexpr (MED == MED_UNIFORM) {
@@ -227,7 +230,8 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     const Real rad = a.source == SRC_DISK ? M<Real>::sqrt(u0 * (R * R))
                                                           : R * M<Real>::sqrt((Real)0.5 * M<Real>::neglog(u0));
                     Real st, ct, sp, cp;
-                    M<Real>::sincos(u1 * TWOPI, &st, &ct);
+                    if constexpr (sizeof(Real) == 8) turn(r.y, st, ct);
+                    else M<Real>::sincos(u1 * TWOPI, &st, &ct);
                     const Real X = rad * ct + K.xmax, Y = rad * st + K.ymax;
                     if constexpr (MED == MED_RHOKAP) {
                         // reference medium: a pure absorber (any interaction
@@ -237,30 +241,38 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                         cp = (Real)1;
                         sp = (Real)0;
                     } else {
-                        if constexpr (SCAT64) turn(s_turn, r.z, sp, cp);
+                        if constexpr (SCAT64) turn(r.z, sp, cp);
                         else M<Real>::sincos(TWOPI * u2, &sp, &cp);
                     }
                     cpv = cp;
                     spv = sp;
                     sint = (Real)0;
-                    if (!(X >= (Real)0 && X < K.w2x && Y >= (Real)0 && Y < K.w2y)) {
+                    if (!(not_negative(X) && less_pos(X, K.w2x) && not_negative(Y) && less_pos(Y, K.w2y))) {
                         atomicAdd(a.tally + T_MISSED, 1.0);
                     } else {
-                        ix = (int)((Real)NX * X / K.w2x);
-                        iy = (int)((Real)NY * Y / K.w2y);
+                        // (FP64: a product; each quotient is ten operations of its pipe)
+                        ix = (int)(sizeof(Real) == 8 ? X * K.cells_x : (Real)NX * X / K.w2x);
+                        iy = (int)(sizeof(Real) == 8 ? Y * K.cells_y : (Real)NY * Y / K.w2y);
                         ix = ix > NX - 1 ? NX - 1 : ix;
                         iy = iy > NY - 1 ? NY - 1 : iy;
                         iz = NZ - 1;
-                        fx = X - (Real)ix * hx;
-                        fy = Y - (Real)iy * hy;
+                        // (straight down: only after a reflection do x and y matter)
+                        if (sizeof(Real) == 4 || a.fresnel || MED != MED_RHOKAP) {
+                            fx = X - (Real)ix * hx;
+                            fy = Y - (Real)iy * hy;
+                        }
                         fz = hz - (Real)1.e-8 * hz;
                         props();
                         w = (Real)1;
                         if (a.fresnel) {
                             const Real nt = MED == MED_RHOKAP ? K.rhokap_n : lut[mid].n;
-                            Real rsp = (namb - nt) / (namb + nt);
-                            rsp = rsp * rsp;
-                            atomicAdd(&s_tal[0], (double)rsp);
+                            Real rsp = K.rhokap_spec;
+                            if constexpr (sizeof(Real) == 4 || MED != MED_RHOKAP) {
+                                rsp = (namb - nt) / (namb + nt);
+                                rsp = rsp * rsp;
+                            }
+                            if constexpr (SPEC_REG) spec += (double)rsp;
+                            else atomicAdd(&s_tal[0], (double)rsp);
                             w = (Real)1 - rsp;
                         }
                         tau = M<Real>::neglog(u3);
@@ -411,6 +423,8 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     // tau holds the flight distance of the interaction point
                     dep += w * (tau - t) * mua;
                     t = tau;
+                } else if constexpr (sizeof(Real) == 8 && MED == MED_RHOKAP) {
+                    dep += w * tau;  // a pure absorber, mua = mut, and the packet ends here
                 } else {
                     const Real dd = M<Real>::div(tau, mut);
                     dep += w * dd * mua;
@@ -525,7 +539,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                             fz = axis_pos(nz, fz, hz, tmz, t);
                             double cost = nz;
                             Azimuth p{cpv, spv};
-                            if (stokes(s_turn, lut[mid].g, lut[mid].g2, r.x, r.y, cost, sint, p)) {
+                            if (stokes(lut[mid].g, lut[mid].g2, r.x, r.y, cost, sint, p)) {
                                 cpv = p.c;
                                 spv = p.s;
                                 nx = sint * cpv;
@@ -553,6 +567,11 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     const unsigned c1 = __reduce_add_sync(FULL, cScat);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cSteps += __shfl_xor_sync(FULL, cSteps, o);
+    if constexpr (SPEC_REG) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) spec += __shfl_xor_sync(FULL, spec, o);
+        if (lane == 0) atomicAdd(&s_tal[0], spec);
+    }
     if (lane == 0) {
         atomicAdd(&s_cnt[1], (unsigned long long)c1);
         atomicAdd(&s_cnt[0], (unsigned long long)cSteps);
@@ -726,6 +745,10 @@ static void fill_consts(TransportArgs &a)
     d.namb = a.n_ambient;
     d.rhokap_n = a.rhokap_n;
     d.src_r = a.source_radius;
+    d.cells_x = a.nx / d.w2x;
+    d.cells_y = a.ny / d.w2y;
+    const double r0 = (d.namb - d.rhokap_n) / (d.namb + d.rhokap_n);
+    d.rhokap_spec = r0 * r0;
     for (int t = 0; t < MAX_MAT; ++t) {
         const OptMat &o = a.lut[t < a.nmat ? t : 0];
         const double mut = o.mua + o.mus, alb = mut > 0.0 ? o.mus / mut : 0.0, g2 = o.g * o.g;

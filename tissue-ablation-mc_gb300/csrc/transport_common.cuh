@@ -16,12 +16,10 @@ namespace {
 // src/constants.f90:13), from a table of 256 steps of the turn and the Taylor terms
 // of the rest, at most 0.0123: next terms 8e-18 and 1e-20.  16 FP64 operations against
 // some 45 of the library's, and the angle itself is never rounded.
-constexpr int TURN = 256;
-__device__ __forceinline__ void turn_table(double2 *tab)
-{
-    for (int i = threadIdx.x; i <= TURN; i += blockDim.x) ::sincos(TWOPI_R * (i * (1.0 / TURN)), &tab[i].x, &tab[i].y);
-}
-__device__ __forceinline__ void turn(const double2 *tab, uint32_t x, double &sn, double &cs)
+static __device__ const double2 g_turn[257] = {
+#include "turn_table.inc"
+};
+__device__ __forceinline__ void turn(uint32_t x, double &sn, double &cs)
 {
     const uint32_t i = ((x >> 23) + 1u) >> 1;
     const int r = (int)(x - (i << 24));
@@ -29,7 +27,7 @@ __device__ __forceinline__ void turn(const double2 *tab, uint32_t x, double &sn,
     const double b = __fma_rn(__hiloint2double(0x43380000 + (r >> 31), r) - 0x1.8p52, k, 0.5 * k), b2 = b * b;
     const double sb = __fma_rn(b * b2, __fma_rn(b2, 1.0 / 120, -1.0 / 6), b);
     const double cm = b2 * __fma_rn(b2, __fma_rn(b2, -1.0 / 720, 1.0 / 24), -0.5);
-    const double2 t = tab[i];
+    const double2 t = g_turn[i];
     sn = t.x + __fma_rn(t.x, cm, t.y * sb);
     cs = t.y + __fma_rn(t.y, cm, -(t.x * sb));
 }
@@ -60,7 +58,7 @@ __device__ __forceinline__ Azimuth mirror_x(Azimuth p)
 // operations; without the acos and that sincos 255: 1e6 packets through a 100^3
 // cube 181 -> 165 ms.  The cosine of the deflection keeps its operations one by one:
 // near +-1 the angle multiplies its last bit by 1e8.
-__device__ __forceinline__ bool stokes(const double2 *tab, double hgg, double g2, uint32_t d0, uint32_t d1, double &cost,
+__device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint32_t d1, double &cost,
                                        double &sint, Azimuth &phi)
 {
     const double u0 = Uniform<double>::from(d0);
@@ -68,7 +66,7 @@ __device__ __forceinline__ bool stokes(const double2 *tab, double hgg, double g2
         cost = 2.0 * u0 - 1.0;
         const double s2 = 1.0 - cost * cost;
         sint = s2 <= 0.0 ? 0.0 : ::sqrt(s2);
-        turn(tab, d1, phi.s, phi.c);
+        turn(d1, phi.s, phi.c);
         return true;
     }
     const double costp = cost, sintp = sint;
@@ -260,6 +258,9 @@ __device__ __forceinline__ bool less_pos(double a, double b)
 {
     return (int64_t)ieee::bits(a) < (int64_t)ieee::bits(b);
 }
+
+__device__ __forceinline__ bool not_negative(float a) { return a >= 0.f; }
+__device__ __forceinline__ bool not_negative(double a) { return (int64_t)ieee::bits(a) >= 0; }
 
 // Per-flight DDA set-up from the in-cell position f and direction n of one
 // axis: td = cell width along the ray, tm = distance to the next face.
