@@ -22,6 +22,7 @@
 // and planes outside the grid are not copied; their cells are read only
 // after the thread that owns the boundary voxel has written its ghost value
 // there.
+#include "f32x2.cuh"
 #include "grid_sync.cuh"
 #include "heat_common.cuh"
 #include "slab_common.cuh"
@@ -731,22 +732,27 @@ __global__ void __launch_bounds__(BP *BR, UNIFORM ? TAM_BSTEP_MINB : 5)
                     knz0 = kc0;
                     knz1 = kc1;
                 }
-                float tn[2], en[2];
+                float2 t2, e2;
+                if (UNIFORM) {
+                    // both voxels at once, each half rounded as the scalar operations
+                    const float2 xm = make_float2(txl, Tc.x), xp = make_float2(Tc.y, txr);
+                    const float2 em = make_float2(exl, Ec.x), eq = make_float2(Ec.y, exr);
+                    const float2 sx = sub2(add2(sub2(xm, Tc), sub2(xp, Tc)), add2(em, eq));
+                    const float2 sy = sub2(add2(sub2(tym, Tc), sub2(typ, Tc)), add2(eym, eyp));
+                    const float2 sz_ = sub2(add2(sub2(Tpz, Tc), sub2(Tnz, Tc)), add2(Epz, Enz));
+                    const float2 dT = fma2(dup(Cz), sz_, fma2(dup(Cy), sy, fma2(dup(Cx), sx, mul2(dup(C6), Ec))));
+                    const float2 yk = sub2(fma2(dup(Ku), j2, dT), Ec);
+                    t2 = add2(Tc, yk);
+                    e2 = sub2(sub2(t2, Tc), yk);
+                } else {
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float tc = h ? Tc.y : Tc.x, e0 = h ? Ec.y : Ec.x;
-                    const float txm = h ? Tc.x : txl, txp = h ? txr : Tc.y, exm = h ? Ec.x : exl, exp_ = h ? exr : Ec.y;
-                    const float tyM = h ? tym.y : tym.x, tyP = h ? typ.y : typ.x;
-                    const float eyM = h ? eym.y : eym.x, eyP = h ? eyp.y : eyp.x;
-                    const float tzM = h ? Tpz.y : Tpz.x, tzP = h ? Tnz.y : Tnz.x, ezM = h ? Epz.y : Epz.x,
-                                ezP = h ? Enz.y : Enz.x;
-                    float dT;
-                    if (UNIFORM) {
-                        const float sx = ((txm - tc) + (txp - tc)) - (exm + exp_);
-                        const float sy = ((tyM - tc) + (tyP - tc)) - (eyM + eyP);
-                        const float sz_ = ((tzM - tc) + (tzP - tc)) - (ezM + ezP);
-                        dT = __fmaf_rn(Cz, sz_, __fmaf_rn(Cy, sy, __fmaf_rn(Cx, sx, C6 * e0)));
-                    } else {
+                    for (int h = 0; h < 2; ++h) {
+                        const float tc = h ? Tc.y : Tc.x, e0 = h ? Ec.y : Ec.x;
+                        const float txm = h ? Tc.x : txl, txp = h ? txr : Tc.y, exm = h ? Ec.x : exl, exp_ = h ? exr : Ec.y;
+                        const float tyM = h ? tym.y : tym.x, tyP = h ? typ.y : typ.x;
+                        const float eyM = h ? eym.y : eym.x, eyP = h ? eyp.y : eyp.x;
+                        const float tzM = h ? Tpz.y : Tpz.x, tzP = h ? Tnz.y : Tnz.x, ezM = h ? Epz.y : Epz.x,
+                                    ezP = h ? Enz.y : Enz.x;
                         const int kk = h ? kc1 : kc0;
                         const unsigned char *SC = S + Lay::C_OFF;
                         const float *frow = L.fa + kk * MAX_MAT;
@@ -756,27 +762,28 @@ __global__ void __launch_bounds__(BP *BR, UNIFORM ? TAM_BSTEP_MINB : 5)
                         const float ayp = cyd * frow[SC[qC + h + RC] & (MAX_MAT - 1)];
                         const float azm = czd * frow[h ? kpz1 : kpz0];
                         const float azp = czd * frow[h ? knz1 : knz0];
-                        dT = ((azm * ((tzM - tc) - (ezM - e0)) + azp * ((tzP - tc) - (ezP - e0))) +
-                              (aym * ((tyM - tc) - (eyM - e0)) + ayp * ((tyP - tc) - (eyP - e0)))) +
-                             (axm * ((txm - tc) - (exm - e0)) + axp * ((txp - tc) - (exp_ - e0)));
+                        const float dT = ((azm * ((tzM - tc) - (ezM - e0)) + azp * ((tzP - tc) - (ezP - e0))) +
+                                          (aym * ((tyM - tc) - (eyM - e0)) + ayp * ((tyP - tc) - (eyP - e0)))) +
+                                         (axm * ((txm - tc) - (exm - e0)) + axp * ((txp - tc) - (exp_ - e0)));
+                        const float Kk = Pdt * L.irc[kk];
+                        const float inc = __fmaf_rn(Kk, h ? j2.y : j2.x, dT);
+                        const float yk = inc - e0;
+                        const float t = tc + yk;
+                        (h ? t2.y : t2.x) = t;
+                        (h ? e2.y : e2.x) = (t - tc) - yk;
                     }
-                    const float Kk = UNIFORM ? Ku : Pdt * L.irc[h ? kc1 : kc0];
-                    const float inc = __fmaf_rn(Kk, h ? j2.y : j2.x, dT);
-                    const float yk = inc - e0;
-                    const float t = tc + yk;
-                    const float e = (t - tc) - yk;
-                    const float tm = tc > t ? tc : t;
-                    if (!(fabsf(tm - lo_t) < lo_t)) fix |= 1u << h;
-                    tn[h] = t;
-                    en[h] = e;
+                }
+                {
+                    const float m0 = Tc.x > t2.x ? Tc.x : t2.x, m1 = Tc.y > t2.y ? Tc.y : t2.y;
+                    fix = (fabsf(m0 - lo_t) < lo_t ? 0u : 1u) | (fabsf(m1 - lo_t) < lo_t ? 0u : 2u);
                 }
                 // rows are not 8-byte aligned in general: scalar stores
                 float *To = d.To + v, *Eo = d.Eo + v;
-                To[0] = tn[0];
-                Eo[0] = en[0];
+                To[0] = t2.x;
+                Eo[0] = e2.x;
                 if (!half) {
-                    To[1] = tn[1];
-                    Eo[1] = en[1];
+                    To[1] = t2.y;
+                    Eo[1] = e2.y;
                 } else {
                     fix &= 1u;
                 }
