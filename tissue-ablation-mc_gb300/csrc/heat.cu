@@ -187,7 +187,7 @@ template <> struct RefOps<float> {
 // (FP64), 24 -> 15 us (FP32, which was bound by the latency of two barriers
 // per plane).  Threads take consecutive columns of the x-y plane, wrapping
 // from row pair to row pair, so no lane idles past a row's end.
-constexpr int REF_TPB = 128, REF_ROWS = 2;
+constexpr int REF_TPB = 128, REF_ROWS = 2, REF_BLOCKS = 6;  // blocks per SM: 80 registers (4: 2 to 6 % slower)
 // a coefficient from the properties of its two cells (rare: kept out of line)
 template <typename F>
 __device__ __noinline__ F ref_face_at(const F *K, const F *Dn, const F *C, uint32_t p, uint32_t q, F id2)
@@ -195,7 +195,7 @@ __device__ __noinline__ F ref_face_at(const F *K, const F *Dn, const F *C, uint3
     return RefOps<F>::face(K[p], K[q], Dn[p], Dn[q], C[p], C[q], id2);
 }
 template <typename F>
-__global__ void __launch_bounds__(REF_TPB, 4) ref_stencil_kernel(const __grid_constant__ RefHeatArgs a0, int zc)
+__global__ void __launch_bounds__(REF_TPB, REF_BLOCKS) ref_stencil_kernel(const __grid_constant__ RefHeatArgs a0, int zc)
 {
     using O = RefOps<F>;
     constexpr int R = REF_ROWS;
@@ -548,7 +548,11 @@ __device__ __noinline__ void damage_props_voxel(const RefArrheniusArgs &d, const
 // that (the general path's compares took 360 instructions per warp; 80^3:
 // 14 -> 9.8 us).  Threads take consecutive cells of a plane, wrapping from row to
 // row.
-__global__ void __launch_bounds__(256) ref_damage_props_kernel(const __grid_constant__ RefArrheniusArgs d,
+// (16 blocks of 128 threads per SM, 32 registers: the rare voxels' code takes 60 and
+// halved the warps that the calm ones' loads are in flight from.  Per iteration of the
+// loop, before: 160^3 FP64 308 -> 290 us, FP32 164 -> 147; 80^3 76.1 -> 75.5)
+constexpr int PROPS_TPB = 128;
+__global__ void __launch_bounds__(PROPS_TPB, 16) ref_damage_props_kernel(const __grid_constant__ RefArrheniusArgs d,
                                                                const __grid_constant__ RefPropsArgs a)
 {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -990,9 +994,14 @@ cudaError_t launch_ref_stencil(const RefHeatArgs &a0, cudaStream_t s)
     a.deltf = (float)a.delt;
     count_launch();
     const int64_t bx = ((int64_t)a.nx * ((a.ny + REF_ROWS - 1) / REF_ROWS) + REF_TPB - 1) / REF_TPB;
-    // columns of 2 to 16 planes, four blocks per SM where the grid allows
-    const int chunks = (int)std::max<int64_t>(1, 152 * 4 / bx);
-    const int zc = std::min(16, std::max(2, (a.nz + chunks - 1) / chunks));
+    // planes per column: the fewest that leave one wave of blocks, at most 3.  Per
+    // iteration of the loop, columns of 1 / 2 / 3 planes and, before, the 2 to 16 of one
+    // wave of four blocks per SM: 40^3 FP64 48.4 / 49.6 / 52.0 and 49.7 us; 80^3 77.3 /
+    // 77.7 / 76.1 and 77.5 (FP32 37.9 / 38.2 / 36.6 and 37.4); 120^3 166 / 160 / 158 and
+    // 163 (87.9 / 81.4 / 83.2 and 87.0); 160^3 308 and 344 (167 and 196)
+    const int64_t wave = 152 * REF_BLOCKS;
+    int zc = std::max(1, (a.nz + 65534) / 65535);
+    while (zc < 3 && bx * ((a.nz + zc - 1) / zc) > wave) ++zc;
     const dim3 grid((unsigned)bx, (a.nz + zc - 1) / zc);
     if (a.f32) ref_stencil_kernel<float><<<grid, REF_TPB, 0, s>>>(a, zc);
     else ref_stencil_kernel<double><<<grid, REF_TPB, 0, s>>>(a, zc);
@@ -1016,8 +1025,8 @@ cudaError_t launch_ref_props(const RefPropsArgs &a, cudaStream_t s)
 cudaError_t launch_ref_damage_props(const RefArrheniusArgs &d, const RefPropsArgs &a, cudaStream_t s)
 {
     count_launch();
-    const unsigned bx = (unsigned)(((int64_t)a.nx * a.ny + 255) / 256);
-    ref_damage_props_kernel<<<dim3(bx, (unsigned)std::min(a.nz, 65535)), 256, 0, s>>>(d, a);
+    const unsigned bx = (unsigned)(((int64_t)a.nx * a.ny + PROPS_TPB - 1) / PROPS_TPB);
+    ref_damage_props_kernel<<<dim3(bx, (unsigned)std::min(a.nz, 65535)), PROPS_TPB, 0, s>>>(d, a);
     return cudaGetLastError();
 }
 
