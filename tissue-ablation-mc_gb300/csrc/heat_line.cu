@@ -17,8 +17,8 @@
 // puts into 4 of 10 warps of a 151-wide row, for the pair at once instead of per
 // voxel: 5 % slower; plane pointers and 32-bit offsets: 4 % slower; scalar
 // arithmetic: 5 % slower.  Per step, staged form before -> now: 151 x 150 x 149
-// 53.8 -> 21.9 us, 101 x 99 x 103 30.4 -> 9.6, 33 x 34 x 35 26.6 -> 6.2; layers
-// 97 x 95 x 60 29.5 -> 8.8, vessels 151 x 140 x 130 49.0 -> 25.1.
+// 53.8 -> 21.6 us, 101 x 99 x 103 30.4 -> 9.3, 33 x 34 x 35 26.6 -> 6.2; layers
+// 97 x 95 x 60 29.5 -> 8.6, vessels 151 x 140 x 130 49.0 -> 24.7.
 #include <algorithm>
 #include <cstring>
 

@@ -353,7 +353,7 @@ def parser():
     h.add_argument("--edge", type=int, default=200)
     h.add_argument("--packets", type=int, default=1_000_000)
     h.add_argument("--steps", type=int, default=4)
-    h.add_argument("--forms", default="slab,pair", help="comma list of slab / pair")
+    h.add_argument("--forms", default="slab,pair", help="comma list of slab (the default quad form) / pair")
     h.add_argument("--geometry", default="cube", choices=["cube", "vessels", "layers"],
                    help="the homogeneous cube, configuration 5's vessels and inclusions at this edge, or "
                         "configuration 3's three-layer slab (edge x edge x edge / 2)")
