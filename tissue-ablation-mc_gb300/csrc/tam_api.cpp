@@ -75,6 +75,8 @@ struct tam_ctx {
     double *d_tally = nullptr;
     unsigned long long *d_work = nullptr, *d_nabl = nullptr, *d_cnt = nullptr;
     double *d_jmean = nullptr, *d_jglob = nullptr, *d_sum = nullptr;
+    bool jraw = false;               // reference loop: the tally awaits its normalisation (by jraw_f) in the next step
+    double jraw_f = 0.0;
     // reference mode
     double *d_T[2] = {nullptr, nullptr};
     int tcur = 0;
@@ -704,8 +706,9 @@ int pass_args(tam_ctx *ctx, int64_t n, uint64_t seed, uint32_t stream, tam::Tran
 }
 
 // Bookkeeping and normalisation (src/mcpolar.f90:174) after a pass's
-// launches on stream s.
-int pass_normalise(tam_ctx *ctx, int64_t n, cudaStream_t s)
+// launches on stream s.  defer (reference mode): left to the stencil of the step
+// that follows at once (ref_heat).
+int pass_normalise(tam_ctx *ctx, int64_t n, cudaStream_t s, bool defer = false)
 {
     ctx->have_mc_time = true;
     ctx->last_n = n;
@@ -722,7 +725,10 @@ int pass_normalise(tam_ctx *ctx, int64_t n, cudaStream_t s)
         const double den = (double)n * (2. * p.xmax * 1.e-2 / p.nxg) * (2. * p.ymax * 1.e-2 / p.nyg) *
                            (2. * p.zmax * 1.e-2 / p.nzg);
         const double f = n > 0 ? (pw / 81.0) / den : 0.0;
-        CK(tam::launch_scale_f64(ctx->d_jglob, ctx->d_jmean, f, ctx->ni, false, s, ctx->d_tally + tam::T_ABSORBED));
+        ctx->jraw = defer;
+        ctx->jraw_f = f;
+        if (!defer)
+            CK(tam::launch_scale_f64(ctx->d_jglob, ctx->d_jmean, f, ctx->ni, false, s, ctx->d_tally + tam::T_ABSORBED));
     }
     ctx->tally_stale = true;
     return TAM_OK;
@@ -731,7 +737,7 @@ int pass_normalise(tam_ctx *ctx, int64_t n, cudaStream_t s)
 // jmean, the tallies and the packet counter behind it
 size_t pass_bytes(const tam_ctx *ctx) { return ((size_t)ctx->ni + tam::N_TALLY + 1) * sizeof(double); }
 
-int mc_pass(tam_ctx *ctx, int64_t n, uint64_t seed, uint32_t stream, bool sync = true)
+int mc_pass(tam_ctx *ctx, int64_t n, uint64_t seed, uint32_t stream, bool sync = true, bool defer = false)
 {
     cudaStream_t s = ctx->stream;
     tam::TransportArgs a;
@@ -753,7 +759,7 @@ int mc_pass(tam_ctx *ctx, int64_t n, uint64_t seed, uint32_t stream, bool sync =
         CK(tam::launch_transport(a, ctx->fp64, ctx->sm_count, s));
     }
     CK(cudaEventRecord(ctx->ev[1], s));
-    RC(pass_normalise(ctx, n, s));
+    RC(pass_normalise(ctx, n, s, defer));
     if (!sync) {
         CK(cudaGetLastError());
         return TAM_OK;
@@ -784,6 +790,8 @@ int ref_classes(tam_ctx *ctx)
 
 int ref_heat(tam_ctx *ctx, int32_t loops)
 {
+    const bool raw = ctx->jraw;  // a pass left its normalisation to this step
+    ctx->jraw = false;
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
     if (ctx->pulseLength < ctx->delt) ctx->delt = ctx->pulseLength / 100.;  // src/3dFD.f90:102-105
     ctx->loops_left = (int)(ctx->total_time / ((double)loops * ctx->delt)) - ctx->counter;
@@ -820,6 +828,12 @@ int ref_heat(tam_ctx *ctx, int32_t loops)
     a.cls = ctx->d_rcls;
     tam::ref_class_faces(a, ctx->rcls);
     for (int32_t it = 0; it < loops; ++it) {
+        if (raw) {
+            a.jraw = it == 0 ? ctx->d_jmean : nullptr;
+            a.jf = ctx->jraw_f;
+            a.jglob = ctx->d_jglob;
+            a.jsum = ctx->d_tally + tam::T_ABSORBED;
+        }
         a.delt = ctx->delt;
         a.laserOn = ctx->laserOn;
         a.t0 = ctx->d_T[ctx->tcur];
@@ -1197,7 +1211,7 @@ int outer_iteration(tam_ctx *ctx, uint64_t seed, bool sync = true)
         RC(cfg_heat(ctx, ctx->p.loops));
     } else {
         // src/mcpolar.f90:149-185
-        if (ctx->laser_flag) RC(mc_pass(ctx, n, seed, (uint32_t)ctx->counter, false));
+        if (ctx->laser_flag) RC(mc_pass(ctx, n, seed, (uint32_t)ctx->counter, false, ctx->p.loops > 0));
         RC(ref_heat(ctx, ctx->p.loops));
         RC(ref_damage_props(ctx, ctx->p.ablate_temp));
         ctx->ref_warm = true;
@@ -2049,9 +2063,7 @@ bool ref_graph_capture(tam_ctx *ctx, uint64_t seed, int slot)
         a.err = ctx->d_err;
         a.work_zeroed = 1;
         ok = cudaMemsetAsync(ctx->d_jmean, 0, pass_bytes(ctx), s) == cudaSuccess &&
-             tam::launch_transport(a, ctx->fp64, ctx->sm_count, s) == cudaSuccess &&
-             tam::launch_scale_f64(ctx->d_jglob, ctx->d_jmean, 0.0, ctx->ni, false, s,
-                                   ctx->d_tally + tam::T_ABSORBED, &iv->f) == cudaSuccess;
+             tam::launch_transport(a, ctx->fp64, ctx->sm_count, s) == cudaSuccess;
         // heat step (src/3dFD.f90:113-187)
         tam::RefHeatArgs h{};
         h.nx = ctx->nx;
@@ -2068,6 +2080,10 @@ bool ref_graph_capture(tam_ctx *ctx, uint64_t seed, int slot)
         h.heatcap = ctx->d_heatcap;
         h.coeff = ctx->d_coeff;
         h.J = ctx->d_jglob;
+        h.jraw = ctx->d_jmean;  // normalised by the step
+        h.jf_dev = &iv->f;
+        h.jglob = ctx->d_jglob;
+        h.jsum = ctx->d_tally + tam::T_ABSORBED;
         h.Q = ctx->d_Q;
         h.err = ctx->d_err;
         h.f32 = ctx->fp64 ? 0 : 1;
@@ -2096,7 +2112,7 @@ bool ref_graph_capture(tam_ctx *ctx, uint64_t seed, int slot)
         ok = ok && tam::launch_ref_damage_props(d, pr, s) == cudaSuccess;
         rcur = 1 - rcur;
     }
-    tam::count_launch(-4 * REF_GRAPH_ITERS);  // captured, not launched (transport, scale, stencil, damage/props)
+    tam::count_launch(-3 * REF_GRAPH_ITERS);  // captured, not launched (transport, stencil, damage/props)
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s, &g);
     ok = ok && e == cudaSuccess && g;
@@ -2166,7 +2182,7 @@ int ref_run(tam_ctx *ctx, uint64_t seed, int64_t max_iters, bool until_time, int
             if (fits) {
                 CK(cudaMemcpyAsync(ctx->d_iv, tab, sizeof tab, cudaMemcpyHostToDevice, ctx->stream));  // pageable: copied now
                 CK(cudaGraphLaunch(ctx->rexec[slot], ctx->stream));
-                tam::count_launch(4 * G);
+                tam::count_launch(3 * G);
                 ctx->counter += G;
                 ctx->mc_passes += G;
                 ctx->last_n = n;

@@ -148,7 +148,7 @@ cudaError_t launch_flush_f32(double *acc, float *part, int nx, int ny, int bx0, 
 // out[q] = in[q] * f for q < n; in is then zeroed when zero_in is set.
 // out = in * f; with `sum`, also *sum += the total of in (the caller zeroes *sum)
 cudaError_t launch_scale_f64(double *out, double *in, double f, int64_t n, bool zero_in, cudaStream_t s,
-                             double *sum = nullptr, const double *f_dev = nullptr);
+                             double *sum = nullptr);
 cudaError_t launch_scale_to_f32(float *out, double *in, double f, int64_t n, bool zero_in, cudaStream_t s,
                                 double *sum = nullptr);
 
@@ -179,6 +179,12 @@ struct RefHeatArgs {
     double *tn;                       // halo, written (interior)
     const double *kappa, *density, *heatcap, *coeff; // halo
     const double *J;                  // interior jmeanGLOBAL
+    // non-null: a pass's tally, normalised by the step (J = jraw * jf, written to jglob;
+    // *jsum += the total of jraw)
+    const double *jraw = nullptr;
+    double jf = 0.0;
+    const double *jf_dev = nullptr;   // non-null: jf is read from here
+    double *jglob = nullptr, *jsum = nullptr;
     double *Q;                        // interior
     unsigned *err;
     int32_t f32;                      // 1: the FP32 form, on the FP32 copies below

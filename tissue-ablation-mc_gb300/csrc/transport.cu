@@ -632,10 +632,8 @@ template <typename Out> __device__ __noinline__ double scale_lit(Out *out, doubl
 // narrow FP64 pipe alone (it bounded this pass; 512,000 cells, 2 % of them lit:
 // 8.6 -> 6.9 us).
 template <typename Out>
-__global__ void scale_kernel(Out *out, double *in, double f, int64_t n, int zero_in, double *sum,
-                             const double *f_dev)
+__global__ void scale_kernel(Out *out, double *in, double f, int64_t n, int zero_in, double *sum)
 {
-    if (f_dev) f = *f_dev;
     const bool plain = ieee::is_finite(f) && ieee::ge_zero(f);
     double acc = 0.0;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
@@ -829,12 +827,11 @@ static int scale_grid(int64_t n)
     return (int)(b > 0 ? b : 1);
 }
 
-cudaError_t launch_scale_f64(double *out, double *in, double f, int64_t n, bool zero_in, cudaStream_t s, double *sum,
-                             const double *f_dev)
+cudaError_t launch_scale_f64(double *out, double *in, double f, int64_t n, bool zero_in, cudaStream_t s, double *sum)
 {
     if (n <= 0) return cudaSuccess;
     count_launch();
-    scale_kernel<double><<<scale_grid(n), 256, 0, s>>>(out, in, f, n, zero_in ? 1 : 0, sum, f_dev);
+    scale_kernel<double><<<scale_grid(n), 256, 0, s>>>(out, in, f, n, zero_in ? 1 : 0, sum);
     return cudaGetLastError();
 }
 
@@ -866,7 +863,7 @@ cudaError_t launch_scale_to_f32(float *out, double *in, double f, int64_t n, boo
 {
     if (n <= 0) return cudaSuccess;
     count_launch();
-    scale_kernel<float><<<scale_grid(n), 256, 0, s>>>(out, in, f, n, zero_in ? 1 : 0, sum, nullptr);
+    scale_kernel<float><<<scale_grid(n), 256, 0, s>>>(out, in, f, n, zero_in ? 1 : 0, sum);
     return cudaGetLastError();
 }
 
