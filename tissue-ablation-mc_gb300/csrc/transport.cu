@@ -426,7 +426,9 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                 } else if constexpr (sizeof(Real) == 8 && MED == MED_RHOKAP) {
                     dep += w * tau;  // a pure absorber, mua = mut, and the packet ends here
                 } else {
-                    const Real dd = M<Real>::div(tau, mut);
+                    Real dd;
+                    if constexpr (sizeof(Real) == 8) dd = div64(tau, mut);
+                    else dd = M<Real>::div(tau, mut);
                     dep += w * dd * mua;
                     t += dd;
                 }
@@ -529,7 +531,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     surface(a.fresnel ? philox4x32_10_rk(ev++, plo, phi32, strm, a.rk).x : 0u);
                 } else {
                     interact();
-                    bool die = !(w > (Real)0);
+                    bool die = sizeof(Real) == 8 ? !ieee::gt_zero((double)w) : !(w > (Real)0);
                     if constexpr (SCAT64) {
                         if (!die) {
                             const U4 r = philox4x32_10_rk(ev++, plo, phi32, strm, a.rk);
@@ -546,13 +548,13 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                                 ny = sint * spv;
                                 nz = cost;
                             }
-                            if (!(nz == nz) || !(nx == nx) || !(ny == ny)) {
+                            if (ieee::is_nan(nz) || ieee::is_nan(nx) || ieee::is_nan(ny)) {
                                 atomicOr(&s_err, (unsigned)DEVERR_NAN);
                                 die = true;
                             } else {
                                 setup();
                                 t = (Real)0;
-                                die = a.roulette && w < wmin && !roulette(r.z);
+                                die = a.roulette && less_pos(w, wmin) && !roulette(r.z);
                                 tau = M<Real>::neglog(Uniform<Real>::from(r.w));
                             }
                         }

@@ -12,6 +12,40 @@
 namespace tam {
 namespace {
 
+// a < b for values that are not negative (nor NaN): FP64 on the bit patterns,
+// which order alike, off GB300's narrow FP64 pipe.
+__device__ __forceinline__ bool less_pos(float a, float b) { return a < b; }
+__device__ __forceinline__ bool less_pos(double a, double b)
+{
+    return (int64_t)ieee::bits(a) < (int64_t)ieee::bits(b);
+}
+
+// FP64 reciprocal and quotient for normal operands: the hardware's approximation
+// (1e-6) and Newton's iteration, the quotient corrected once by its remainder
+// (Markstein, 1990).  No special cases and no call, 4 and 6 operations of the FP64 pipe;
+// the same bits as IEEE division for all of 2e8 pairs over 1e-280 to 1e280.
+__device__ __forceinline__ double rcp_seed(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+__device__ __forceinline__ double rcp64(double x)
+{
+    double y = rcp_seed(x);
+    y = __fma_rn(y, __fma_rn(-x, y, 1.0), y);
+    return __fma_rn(y, __fma_rn(-x, y, 1.0), y);
+}
+__device__ __forceinline__ double div64(double a, double b)
+{
+    const double y0 = rcp_seed(b), e = __fma_rn(-b, y0, 1.0), y = __fma_rn(y0, __fma_rn(e, e, e), y0), q = a * y;
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// |a| > 1, |a| < 1 and the sign, off the FP64 pipe (a NaN counts as neither)
+__device__ __forceinline__ bool above_one(double a) { return (ieee::bits(a) & ~ieee::SIGN) - (ieee::ONE + 1) < ieee::PINF - ieee::ONE; }
+__device__ __forceinline__ bool below_one(double a) { return (ieee::bits(a) & ~ieee::SIGN) < ieee::ONE; }
+__device__ __forceinline__ bool is_minus(double a) { return (int64_t)ieee::bits(a) < 0; }
+
 // (sin, cos) of TWOPI u, u = (x + 1/2) 2^-32 (TWOPI: the truncated constant of
 // src/constants.f90:13), from a table of 256 steps of the turn and the Taylor terms
 // of the rest, at most 0.0123: next terms 8e-18 and 1e-20.  16 FP64 operations against
@@ -70,27 +104,23 @@ __device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint3
         return true;
     }
     const double costp = cost, sintp = sint;
-    const double t = (1.0 - g2) / (1.0 - hgg + 2.0 * hgg * u0);
-    double bmu = ((1.0 + g2) - t * t) / (2.0 * hgg);
-    double cosb2 = bmu * bmu;
-    if (fabs(bmu) > 1.0) {
-        bmu = bmu > 1.0 ? 1.0 : -1.0;
-        cosb2 = 1.0;
-    }
-    if (bmu == 1.0 || bmu == -1.0) return false;  // direction unchanged
+    const double t = div64(1.0 - g2, 1.0 - hgg + 2.0 * hgg * u0);
+    const double bmu = ((1.0 + g2) - t * t) / (2.0 * hgg);
+    const double cosb2 = bmu * bmu;
+    if (above_one(bmu) || (ieee::bits(bmu) & ~ieee::SIGN) == ieee::ONE) return false;  // direction unchanged
     const double sinbt = ::sqrt(1.0 - cosb2);
     const double ri1 = TWOPI_R * Uniform<double>::from(d1);
-    const bool upper = ri1 > PI_R;
+    const bool upper = less_pos(PI_R, ri1);
     const double ang = upper ? TWOPI_R - ri1 : ri1;
     double sa, ca;
     ::sincos(ang, &sa, &ca);
     double cosi2 = 0.0, sini2;
     cost = costp * bmu + sintp * sinbt * ca;
-    if (fabs(cost) < 1.0) {
+    if (below_one(cost)) {
         sint = fabs(::sqrt(1.0 - cost * cost));
-        sini2 = sa * sintp / sint;
+        sini2 = div64(sa * sintp, sint);
         const double bott = sint * sinbt;
-        cosi2 = costp / bott - cost * bmu / bott;
+        cosi2 = div64(costp, bott) - div64(cost * bmu, bott);
     } else {
         sint = 0.0;
         sini2 = 0.0;
@@ -98,16 +128,15 @@ __device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint3
         if (cost <= -1.0) cosi2 = 1.0;
     }
     double cd = -cosi2 * ca + sini2 * sa * bmu;
-    if (fabs(cd) > 1.0) cd = cd > 1.0 ? 1.0 : -1.0;
+    if (above_one(cd)) cd = is_minus(cd) ? -1.0 : 1.0;
     double sd = ::sqrt((1.0 - cd) * (1.0 + cd));
     sd = upper ? sd : -sd;
     const Azimuth p = phi;
     phi = turned(p, cd, sd);
     // above TWOPI: minus TWOPI; below 0: plus TWOPI (a turn by up to PI from [0, TWOPI])
-    bool over = phi.s > SIN_2PI && phi.c > 0.0 && (p.s < 0.0 || phi.s < 0.0);
-    over = upper && (over || (p.s < 0.0 && phi.s >= 0.0));
-    if (over) phi = turned(phi, COS_2PI, -SIN_2PI);
-    else if (!upper && p.s >= 0.0 && phi.s < 0.0) phi = turned(phi, COS_2PI, SIN_2PI);
+    const bool low0 = is_minus(p.s), low = is_minus(phi.s), near = low && less_pos(-phi.s, -SIN_2PI);
+    if (upper ? (low0 && !low) || (near && !is_minus(phi.c)) : !low0 && low)
+        phi = turned(phi, COS_2PI, upper ? -SIN_2PI : SIN_2PI);
     // back to length 1 (one Newton step)
     const double k = 1.5 - 0.5 * (phi.c * phi.c + phi.s * phi.s);
     phi.c *= k;
@@ -251,14 +280,6 @@ inline int packets_per_warp(int64_t n, int64_t warps)
     return (int)(k < 1 ? 1 : (k > 32 ? 32 : k));
 }
 
-// a < b for values that are not negative (nor NaN): FP64 on the bit patterns,
-// which order alike, off GB300's narrow FP64 pipe.
-__device__ __forceinline__ bool less_pos(float a, float b) { return a < b; }
-__device__ __forceinline__ bool less_pos(double a, double b)
-{
-    return (int64_t)ieee::bits(a) < (int64_t)ieee::bits(b);
-}
-
 __device__ __forceinline__ bool not_negative(float a) { return a >= 0.f; }
 __device__ __forceinline__ bool not_negative(double a) { return (int64_t)ieee::bits(a) >= 0; }
 
@@ -281,6 +302,19 @@ __device__ __forceinline__ void axis_setup(Real n, Real f, Real h, Real BIG, Rea
     tm = tm < (Real)0 ? (Real)0 : tm;
     sg = n > (Real)0 ? 1 : -1;
 }
+// FP64: no compare and no division with special cases; |n| below 1e-289 counts as
+// parallel to the faces.
+__device__ __forceinline__ bool parallel64(double n) { return (__double2hiint(n) & 0x7fffffff) < 0x03e00000; }
+template <>
+__device__ __forceinline__ void axis_setup<double>(double n, double f, double h, double BIG, double &td, double &tm, int &sg)
+{
+    const bool par = parallel64(n), minus = is_minus(n);
+    const double inv = rcp64(n);
+    const double to = (minus ? -f : h - f) * inv;
+    td = par ? BIG : h * fabs(inv);
+    tm = par ? BIG : (is_minus(to) ? 0.0 : to);
+    sg = par || minus ? -1 : 1;
+}
 // FP32: approximate reciprocal; |n| below 1e-30 counts as parallel to the
 // faces (its reciprocal would overflow and turn 0 * inf into NaN).
 template <>
@@ -299,6 +333,12 @@ template <typename Real> __device__ __forceinline__ Real axis_pos(Real n, Real f
 {
     const Real r = n > (Real)0 ? h - (tm - t) * n : (n < (Real)0 ? -(tm - t) * n : f);
     return clamp0h(r, h);
+}
+template <> __device__ __forceinline__ double axis_pos<double>(double n, double f, double h, double tm, double t)
+{
+    const bool minus = is_minus(n);
+    const double d = tm - t, r = parallel64(n) ? f : __fma_rn(-d, n, minus ? 0.0 : h);
+    return is_minus(r) ? 0.0 : (less_pos(h, r) ? h : r);
 }
 
 // VSTEPS voxel steps (src/inttau2.f90:37-63) of the FP32 distance-tracked
