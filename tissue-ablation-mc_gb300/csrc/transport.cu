@@ -227,8 +227,11 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     const Real u0 = Uniform<Real>::from(r.x), u1 = Uniform<Real>::from(r.y);
                     const Real u2 = Uniform<Real>::from(r.z), u3 = Uniform<Real>::from(r.w);
                     const Real R = K.src_r;
-                    const Real rad = a.source == SRC_DISK ? M<Real>::sqrt(u0 * (R * R))
-                                                          : R * M<Real>::sqrt((Real)0.5 * M<Real>::neglog(u0));
+                    auto root = [](Real x) {
+                        if constexpr (sizeof(Real) == 8) return sqrt64(x);
+                        else return M<Real>::sqrt(x);
+                    };
+                    const Real rad = a.source == SRC_DISK ? root(u0 * (R * R)) : R * root((Real)0.5 * M<Real>::neglog(u0));
                     Real st, ct, sp, cp;
                     if constexpr (sizeof(Real) == 8) turn(r.y, st, ct);
                     else M<Real>::sincos(u1 * TWOPI, &st, &ct);

@@ -41,6 +41,22 @@ __device__ __forceinline__ double div64(double a, double b)
     const double y0 = rcp_seed(b), e = __fma_rn(-b, y0, 1.0), y = __fma_rn(y0, __fma_rn(e, e, e), y0), q = a * y;
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
+// |n| below 1e-289, where the reciprocal leaves the normal numbers
+__device__ __forceinline__ bool is_tiny(double n) { return (__double2hiint(n) & 0x7fffffff) < 0x03e00000; }
+// Square root of a normal operand or zero: g -> sqrt(x) and h -> 1 / (2 sqrt(x)) together
+// from the hardware's approximation (Goldschmidt), then one correction by the remainder
+// (Markstein): 7 operations, the bits of the IEEE square root for all of 2e8 operands.
+__device__ __forceinline__ double sqrt64(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    const double r = __fma_rn(-h, g, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    g = __fma_rn(__fma_rn(-g, g, x), h, g);
+    return ieee::is_zero(x) ? x : g;
+}
 // |a| > 1, |a| < 1 and the sign, off the FP64 pipe (a NaN counts as neither)
 __device__ __forceinline__ bool above_one(double a) { return (ieee::bits(a) & ~ieee::SIGN) - (ieee::ONE + 1) < ieee::PINF - ieee::ONE; }
 __device__ __forceinline__ bool below_one(double a) { return (ieee::bits(a) & ~ieee::SIGN) < ieee::ONE; }
@@ -99,16 +115,17 @@ __device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint3
     if (hgg == 0.0) {
         cost = 2.0 * u0 - 1.0;
         const double s2 = 1.0 - cost * cost;
-        sint = s2 <= 0.0 ? 0.0 : ::sqrt(s2);
+        sint = s2 <= 0.0 ? 0.0 : sqrt64(s2);
         turn(d1, phi.s, phi.c);
         return true;
     }
     const double costp = cost, sintp = sint;
     const double t = div64(1.0 - g2, 1.0 - hgg + 2.0 * hgg * u0);
-    const double bmu = ((1.0 + g2) - t * t) / (2.0 * hgg);
+    const double num = (1.0 + g2) - t * t;
+    const double bmu = is_tiny(hgg) ? num / (2.0 * hgg) : div64(num, 2.0 * hgg);
     const double cosb2 = bmu * bmu;
     if (above_one(bmu) || (ieee::bits(bmu) & ~ieee::SIGN) == ieee::ONE) return false;  // direction unchanged
-    const double sinbt = ::sqrt(1.0 - cosb2);
+    const double sinbt = sqrt64(1.0 - cosb2);
     const double ri1 = TWOPI_R * Uniform<double>::from(d1);
     const bool upper = less_pos(PI_R, ri1);
     const double ang = upper ? TWOPI_R - ri1 : ri1;
@@ -117,7 +134,7 @@ __device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint3
     double cosi2 = 0.0, sini2;
     cost = costp * bmu + sintp * sinbt * ca;
     if (below_one(cost)) {
-        sint = fabs(::sqrt(1.0 - cost * cost));
+        sint = sqrt64(1.0 - cost * cost);
         sini2 = div64(sa * sintp, sint);
         const double bott = sint * sinbt;
         cosi2 = div64(costp, bott) - div64(cost * bmu, bott);
@@ -129,7 +146,7 @@ __device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint3
     }
     double cd = -cosi2 * ca + sini2 * sa * bmu;
     if (above_one(cd)) cd = is_minus(cd) ? -1.0 : 1.0;
-    double sd = ::sqrt((1.0 - cd) * (1.0 + cd));
+    double sd = sqrt64((1.0 - cd) * (1.0 + cd));
     sd = upper ? sd : -sd;
     const Azimuth p = phi;
     phi = turned(p, cd, sd);
@@ -302,13 +319,12 @@ __device__ __forceinline__ void axis_setup(Real n, Real f, Real h, Real BIG, Rea
     tm = tm < (Real)0 ? (Real)0 : tm;
     sg = n > (Real)0 ? 1 : -1;
 }
-// FP64: no compare and no division with special cases; |n| below 1e-289 counts as
+// FP64: no compare and no division with special cases; a tiny |n| counts as
 // parallel to the faces.
-__device__ __forceinline__ bool parallel64(double n) { return (__double2hiint(n) & 0x7fffffff) < 0x03e00000; }
 template <>
 __device__ __forceinline__ void axis_setup<double>(double n, double f, double h, double BIG, double &td, double &tm, int &sg)
 {
-    const bool par = parallel64(n), minus = is_minus(n);
+    const bool par = is_tiny(n), minus = is_minus(n);
     const double inv = rcp64(n);
     const double to = (minus ? -f : h - f) * inv;
     td = par ? BIG : h * fabs(inv);
@@ -337,7 +353,7 @@ template <typename Real> __device__ __forceinline__ Real axis_pos(Real n, Real f
 template <> __device__ __forceinline__ double axis_pos<double>(double n, double f, double h, double tm, double t)
 {
     const bool minus = is_minus(n);
-    const double d = tm - t, r = parallel64(n) ? f : __fma_rn(-d, n, minus ? 0.0 : h);
+    const double d = tm - t, r = is_tiny(n) ? f : __fma_rn(-d, n, minus ? 0.0 : h);
     return is_minus(r) ? 0.0 : (less_pos(h, r) ? h : r);
 }
 
