@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
         // ------------------------------------------------- flight phase --
         // voxel steps of the flying lanes until enough lanes wait for the
         // event batch or none flies
-        Real tmin, ahead;
+        Real tmin, ahead, gap;
         bool px = false, py = false, pz = false;  // FP64: the axis of the next face
         // whether the flight's interaction point lies beyond the next face
         // (ties between faces go z over y over x, src/inttau2.f90:116-118)
@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                 py = yz && !px;
                 pz = !yz && !px;
             }
-            ahead = DIST ? tmin : (tmin - t) * mut;  // distance, or optical depth to the face
+            gap = tmin - t;
+            ahead = DIST ? tmin : gap * mut;  // distance, or optical depth to the face
             return less_pos(ahead, tau);
         };
         bool go = look() && alive, capped = false;
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                     go = false;
                 }
             }
-            const Real d = dep + w * (tmin - t) * mua;
+            const Real d = dep + w * (sizeof(Real) == 8 ? gap : tmin - t) * mua;
             if (go) deposit<T32>(a, cell(), ix, iy, iz, d);
             // step into the next cell, branch-free over the axis; the
             // reference snaps the crossed coordinate to the face +- delta
@@ -350,9 +351,12 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                 tau = go ? tau - ahead : tau;
                 t = go ? tmin : t;
                 const bool cx = go && px, cy = go && py, cz = go && pz;
-                tmx = cx ? tmx + (NUDGE ? tdx * knx : tdx) : tmx;
-                tmy = cy ? tmy + (NUDGE ? tdy * kny : tdy) : tmy;
-                tmz = cz ? tmz + (NUDGE ? tdz * knz : tdz) : tmz;
+                // (the crossed axis chosen first: one FP64 addition, not three)
+                const Real td = px ? tdx : (py ? tdy : tdz);
+                const Real next = tmin + (NUDGE ? td * (px ? knx : (py ? kny : knz)) : td);
+                tmx = cx ? next : tmx;
+                tmy = cy ? next : tmy;
+                tmz = cz ? next : tmz;
                 ix += cx ? sgx : 0;
                 iy += cy ? sgy : 0;
                 iz += cz ? sgz : 0;
