@@ -106,7 +106,7 @@ struct tam_ctx {
     bool shadow_ok = false;
 
     // tuning knobs
-    int scat_min = 20;
+    int scat_min = tam::SCAT_MIN;
     int tally32 = -1;                // FP32 transport: -1 auto (FP32 tally when the FP64 one exceeds 256 MB), 0 off, 1 on
     int bricks = -1;                 // material lookups through the brick table: -1 auto (grids of 2^25 voxels
                                      // and more), 0 off, 1 on
@@ -1565,6 +1565,7 @@ int tam_create(const tam_params *p, const tam_config *cfg, tam_ctx **out)
     ctx->config = p->mode == TAM_MODE_CONFIG;
     if (ctx->config) ctx->cfg = *cfg;
     ctx->fp64 = p->precision == TAM_FP64;
+    ctx->scat_min = ctx->fp64 ? tam::SCAT_MIN64 : tam::SCAT_MIN;
     ctx->device = p->device;
     ctx->nx = p->nxg;
     ctx->ny = p->nyg;

@@ -57,6 +57,13 @@ template <typename Real> struct TrConst {
     Real rhokap_spec;                 // normal reflectance of the rhokap medium
 };
 
+// Lanes of a warp that wait before an event batch.  FP64: an event's warp
+// instructions cost the FP64 pipe the same for one lane as for 32, a voxel step is
+// short and taken singly (20 with four steps per pair of votes, the FP32 form's best:
+// 1e6 packets through a 100^3 cube 120 against 114 ms; 16 / 24 / 28 / 32 singly: 83 /
+// 72 / 69 / 69 per 5e5).
+constexpr int SCAT_MIN = 20, SCAT_MIN64 = 30;
+
 // One material's optics in the transport's precision.
 template <typename Real> struct MatR {
     Real mut, mua, alb, g, g2, n;

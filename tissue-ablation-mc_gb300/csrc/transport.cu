@@ -104,7 +104,7 @@ __device__ __forceinline__ void fetch(const TransportArgs &a, const MatR<Real> *
 // nested branches (5491 -> about 3900 warp instructions per packet); 47 against
 // 64 ms per 1e7 packets on the three-layer slab, 154 against 192 ms on a 384^3
 // vessel grid.  scat_min 12 to 24 are within 1 % of each other; 2, 3 and 6
-// voxel steps per vote are 5, 3 and 2 % slower than 4.
+// voxel steps per vote are 5, 3 and 2 % slower than 4.  FP64: see SCAT_MIN64.
 //
 // The DDA is incremental (Amanatides & Woo): per flight, the distance tm to
 // the next face of each axis and the cell width td along the ray; a crossing
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                         go = g != 0;
                     } else {
 #pragma unroll
-                        for (int q = 0; q < (MED == MED_RHOKAP ? 1 : VSTEPS); ++q) vstep(std::false_type{});
+                        for (int q = 0; q < (MED == MED_RHOKAP || sizeof(Real) == 8 ? 1 : VSTEPS); ++q) vstep(std::false_type{});
                     }
                 }
             } else {
@@ -717,7 +717,7 @@ cudaError_t launch_t(const TransportArgs &a, int sm_count, cudaStream_t s)
 {
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, transport_kernel<Real, MED, T32>, TPB, 0);
-    const int scat_min = a.scat_min > 0 ? a.scat_min : 20;
+    const int scat_min = a.scat_min > 0 ? a.scat_min : (sizeof(Real) == 8 ? SCAT_MIN64 : SCAT_MIN);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     const int per_warp = packets_per_warp(a.n, (int64_t)sm_count * (TPB / 32));
