@@ -104,10 +104,10 @@ __device__ __forceinline__ Azimuth mirror_x(Azimuth p)
 // The reference wraps phi by the truncated TWOPI, a turn of 3e-7: wrapped here at the
 // same angles.
 //
-// The FP64 pipe bounds the walk (83 % busy), and a scatter took some 310 of its
-// operations; without the acos and that sincos 255 (1e6 packets through a 100^3 cube
-// 181 -> 165 ms), with quotients and roots of their own and compares on the bits 200
-// (123 ms).  The cosine of the deflection keeps its operations one by one: near +-1
+// The FP64 pipe bounds the walk (83 % busy).  A pass of 2e5 packets through a 100^3
+// cube (3.9e7 scatters, 9.7e7 voxel steps) took 1.385e10 of its operations, without
+// the acos and that sincos 1.288e10 (1e6 packets 181 -> 165 ms), with quotients and
+// roots of their own and compares on the bits 1.032e10 (123 ms).  The cosine of the deflection keeps its operations one by one: near +-1
 // the angle multiplies its last bit by 1e8.
 __device__ __forceinline__ bool stokes(double hgg, double g2, uint32_t d0, uint32_t d1, double &cost,
                                        double &sint, Azimuth &phi)
