@@ -87,9 +87,12 @@ __global__ void __launch_bounds__(TPB64) cls64_step_kernel(const __grid_constant
     const double Cx = cxd * au, Cy = cyd * au, Cz = czd * au, Ku = Pdt * L.irc[uc];
     // screens on the bit patterns, which order like the values they are
     // compared with: at or above them lie the listed temperatures and the
-    // negative and NaN ones
-    const uint64_t screen = ieee::bits(a.dc[FC_SCREEN]);
-    const uint64_t boil = a.boil ? ieee::bits(a.dc[FC_TBOIL]) : ~0ull;
+    // negative and NaN ones.  That holds from +0 up: a screen below (T_lo = 0 K,
+    // 0.01 K below which it lies) or NaN becomes +0, which takes every voxel, and
+    // the exact tests decide
+    auto word = [](double s) -> uint64_t { return ieee::gt_zero(s) ? ieee::bits(s) : 0; };
+    const uint64_t screen = word(a.dc[FC_SCREEN]);
+    const uint64_t boil = a.boil ? word(a.dc[FC_TBOIL]) : ~0ull;
     auto klass = [&](int64_t q) -> int { return UNIFORM ? uc : (int)__ldg(cls + q); };
     // difference towards the neighbour n across face f, or the face's ghost
     // (Dirichlet: the face's temperature; Robin: -h d / k (T - T_amb)); in a

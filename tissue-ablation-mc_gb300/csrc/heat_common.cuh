@@ -54,6 +54,17 @@ template <typename Real> __device__ __forceinline__ Real step_pdt(const FusedArg
 }
 __device__ __forceinline__ double step_tnew(const FusedArgs &a) { return a.sv ? a.sv->t_new : a.t_new; }
 
+// The one screen of the listed rare work of the quad and line forms: damage or
+// ablation, and boiling.  They compare temperatures with it as unsigned words,
+// which order like the values only from +0 up, so a screen below that (T_lo = 0 K,
+// 0.01 K below which the screen lies) or NaN lists every voxel.
+inline float rare_screen(const FusedArgs &a)
+{
+    float s = a.fc[FC_SCREEN];
+    if (a.boil && a.fc[FC_TBOIL] < s) s = a.fc[FC_TBOIL];
+    return s > 0.f ? s : 0.f;
+}
+
 // Laplacian term of one boundary face f (x-, x+, y-, y+, z-, z+): the ghost
 // carries the voxel's own properties, so the face diffusivity is k/(rho c);
 // (ghost - true centre) is the Dirichlet value minus the true temperature, or

@@ -288,9 +288,7 @@ cudaError_t launch_line_step(const FusedArgs &a0, const ClassLut &L, const uint8
 {
     FusedArgs a = a0;
     fill_fused_consts(a);
-    // one screen for the listed rare work: damage / ablation, and boiling
-    float rare_thr = a.fc[FC_SCREEN];
-    if (a.boil && a.fc[FC_TBOIL] < rare_thr) rare_thr = a.fc[FC_TBOIL];
+    const float rare_thr = rare_screen(a);
     LineFaces F{};
     for (int f = 0; f < 6; ++f)
         for (int c = 0; c < MAX_MAT; ++c) {

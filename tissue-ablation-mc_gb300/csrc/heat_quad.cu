@@ -484,9 +484,7 @@ cudaError_t launch_quad_step(const FusedArgs &a0, const ClassLut &L, const uint8
 {
     FusedArgs a = a0;
     fill_fused_consts(a);
-    // one screen for the listed rare work: damage / ablation, and boiling
-    float rare_thr = a.fc[FC_SCREEN];
-    if (a.boil && a.fc[FC_TBOIL] < rare_thr) rare_thr = a.fc[FC_TBOIL];
+    const float rare_thr = rare_screen(a);
     const int bx = (int)(((int64_t)(a.nx / 4) * a.ny + QTPB - 1) / QTPB);
     // planes per block: as many as leave 5000 blocks (four waves), at most 5.
     // Per step with a core in the damage window, 1 / 2 / 3 / 4 / 6 planes: 64^3 5.7 /
