@@ -199,9 +199,7 @@ __global__ void __launch_bounds__(BP *BR, bslab_minb(UNIFORM))
             const float Ku = Pdt * L.irc[uc];
             const unsigned exy = (unsigned)(x == 0) | (unsigned)(x + 1 == nx - 1) << 1 | (unsigned)(y == 0) << 2 |
                                  (unsigned)(y == ny - 1) << 3;
-            float rare_thr = A.fc[FC_SCREEN];
-            if (A.boil && A.fc[FC_TBOIL] < rare_thr) rare_thr = A.fc[FC_TBOIL];
-            const float lo_t = 0.5f * rare_thr;  // new temperatures outside (0, rare_thr) are listed
+            const unsigned thr = __float_as_uint(rare_screen(A));
 
             // planes idx = 0 .. last (z = z0 - 1 .. z1): rows y0 - 1 .. y0 + 8 of T and
             // the Kahan term (11 chunks each), rows y0 .. y0 + 7 of J for the item's
@@ -408,8 +406,7 @@ __global__ void __launch_bounds__(BP *BR, bslab_minb(UNIFORM))
                     const float yk = inc - e0;
                     const float t = tc + yk;
                     const float e = (t - tc) - yk;
-                    const float tm = tc > t ? tc : t;
-                    if (!(fabsf(tm - lo_t) < lo_t)) fix |= 1u << h;
+                    if (hot_word(tc, t) >= thr) fix |= 1u << h;
                     tn[h] = t;
                     en[h] = e;
                 }
@@ -555,9 +552,7 @@ __global__ void __launch_bounds__(BP *BR, UNIFORM ? TAM_BSTEP_MINB : 5)
             const float Ku = Pdt * L.irc[uc];
             const unsigned exy = (unsigned)(x == 0) | (unsigned)(x + 1 == nx - 1) << 1 | (unsigned)(y == 0) << 2 |
                                  (unsigned)(y == ny - 1) << 3;
-            float rare_thr = A.fc[FC_SCREEN];
-            if (A.boil && A.fc[FC_TBOIL] < rare_thr) rare_thr = A.fc[FC_TBOIL];
-            const float lo_t = 0.5f * rare_thr;  // new temperatures outside (0, rare_thr) are marked
+            const unsigned thr = __float_as_uint(rare_screen(A));
 
             // planes idx = 0 .. last (z = z0 - 1 .. z1): rows y0 - 1 .. y0 + 8 of T and
             // the Kahan term (11 chunks each), rows y0 .. y0 + 7 of J for the item's
@@ -773,10 +768,7 @@ __global__ void __launch_bounds__(BP *BR, UNIFORM ? TAM_BSTEP_MINB : 5)
                         (h ? e2.y : e2.x) = (t - tc) - yk;
                     }
                 }
-                {
-                    const float m0 = Tc.x > t2.x ? Tc.x : t2.x, m1 = Tc.y > t2.y ? Tc.y : t2.y;
-                    fix = (fabsf(m0 - lo_t) < lo_t ? 0u : 1u) | (fabsf(m1 - lo_t) < lo_t ? 0u : 2u);
-                }
+                fix = (hot_word(Tc.x, t2.x) >= thr ? 1u : 0u) | (hot_word(Tc.y, t2.y) >= thr ? 2u : 0u);
                 // rows are not 8-byte aligned in general: scalar stores
                 float *To = d.To + v, *Eo = d.Eo + v;
                 To[0] = t2.x;

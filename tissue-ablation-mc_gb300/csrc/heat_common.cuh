@@ -54,16 +54,20 @@ template <typename Real> __device__ __forceinline__ Real step_pdt(const FusedArg
 }
 __device__ __forceinline__ double step_tnew(const FusedArgs &a) { return a.sv ? a.sv->t_new : a.t_new; }
 
-// The one screen of the listed rare work of the quad and line forms: damage or
-// ablation, and boiling.  They compare temperatures with it as unsigned words,
-// which order like the values only from +0 up, so a screen below that (T_lo = 0 K,
-// 0.01 K below which the screen lies) or NaN lists every voxel.
-inline float rare_screen(const FusedArgs &a)
+// The one screen of the rare work that the quad, line and batched slab forms list
+// voxels for: damage or ablation, and boiling.  A voxel is listed when the larger
+// of its old and new temperature, as unsigned words, reaches the screen's: the
+// words order like the values from +0 up, and the negative and NaN ones lie above
+// them all.  So a screen below +0 (T_lo = 0 K, 0.01 K below which it lies) or NaN
+// becomes +0, which lists every voxel.
+__host__ __device__ inline float rare_screen(const FusedArgs &a)
 {
     float s = a.fc[FC_SCREEN];
     if (a.boil && a.fc[FC_TBOIL] < s) s = a.fc[FC_TBOIL];
     return s > 0.f ? s : 0.f;
 }
+
+__device__ __forceinline__ unsigned hot_word(float t0, float t1) { return max(__float_as_uint(t0), __float_as_uint(t1)); }
 
 // Laplacian term of one boundary face f (x-, x+, y-, y+, z-, z+): the ghost
 // carries the voxel's own properties, so the face diffusivity is k/(rho c);

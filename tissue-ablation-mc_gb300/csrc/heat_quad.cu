@@ -240,7 +240,6 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
     float *To = (float *)a.T_out, *Eo = a.Tc_out;
     const int uc = L.uniform >= 0 ? L.uniform : 0;
     const unsigned thr = __float_as_uint(rare_thr);
-    const float lo = 0.5f * rare_thr;
     const bool act = y < ny;
     const int lane = threadIdx.x & 31;
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -332,19 +331,13 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
             if (act && (!HET || st != 0xFF)) {
                 *reinterpret_cast<float4 *>(To + v) = make_float4(t0.x, t0.y, t1.x, t1.y);
                 *reinterpret_cast<float4 *>(Eo + v) = make_float4(e0.x, e0.y, e1.x, e1.y);
-                // listed: an old or new temperature at the screen, or a new one
-                // negative or NaN.  As unsigned words these are the large ones: one
-                // test for the quad first
-                auto u = [](float f) { return __float_as_uint(f); };
-                const unsigned m = max(max(max(u(tc.x), u(tc.y)), max(u(tc.z), u(tc.w))), max(max(u(t0.x), u(t0.y)), max(u(t1.x), u(t1.y))));
-                if (m >= thr) {
-                    const float c4[4] = {tc.x, tc.y, tc.z, tc.w}, t4[4] = {t0.x, t0.y, t1.x, t1.y};
+                // listed: an old or new temperature at the screen, negative or NaN
+                // (rare_screen), one test for the quad first
+                const unsigned m4[4] = {hot_word(tc.x, t0.x), hot_word(tc.y, t0.y), hot_word(tc.z, t1.x), hot_word(tc.w, t1.y)};
+                if (max(max(m4[0], m4[1]), max(m4[2], m4[3])) >= thr) {
                     unsigned fix = 0;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float mm = c4[k] > t4[k] ? c4[k] : t4[k];
-                        if (!(fabsf(mm - lo) < lo)) fix |= 1u << k;
-                    }
+                    for (int k = 0; k < 4; ++k) fix |= (m4[k] >= thr ? 1u : 0u) << k;
                     int at = atomicAdd(&s_cnt, __popc(fix));
                     const int l = ((z - z0) * QTPB + (int)threadIdx.x) * 4;
 #pragma unroll
@@ -399,8 +392,7 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
             const float yk = inc - e0, t = tc + yk;
             To[v] = t;
             Eo[v] = (t - tc) - yk;
-            const float mm = tc > t ? tc : t;
-            if (!(fabsf(mm - lo) < lo)) s_list[atomicAdd(&s_cnt, 1)] = (unsigned short)(4 * l + (n & 3));
+            if (hot_word(tc, t) >= thr) s_list[atomicAdd(&s_cnt, 1)] = (unsigned short)(4 * l + (n & 3));
         }
         if (nf) __syncthreads();
     }
