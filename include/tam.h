@@ -297,6 +297,8 @@ int tam_get_timing(struct tam_ctx *ctx, double *transport_ms, double *heat_ms, i
  * never, 1 always; same walks either way), "heat.zchunk" (z planes per
  * thread column of the fused step, 0 = automatic; on a grid of several
  * thermal classes the next heat call rebuilds the quad form's class table),
+ * "heat.zauto" (1: automatic whatever "heat.zchunk" holds, until that is set
+ * again; 0, the default: as "heat.zchunk" says),
  * "heat.tma" (1: stage the FP32 fused step's planes with TMA, or run the quad
  * form, where the row pitch allows; 0: the line form, or cp.async),
  * "heat.cls" (1: while the thermal properties are those of the material
@@ -387,8 +389,10 @@ int tam_load_state(struct tam_ctx *ctx, const char *path);
  * `packets`) and of "heat.zchunk" / "heat.slab" / "heat.cls_rows" (`steps`
  * heat steps), keeps the fastest and puts the context's state back as it was
  * (fields, clock, pulse state, tallies).  0 packets or 0 steps skips that
- * part.  chosen (nullable) receives up to nchosen values: scat_min, zchunk,
- * cls_rows, slab.
+ * part.  The settings in force are timed too and stay unless others are
+ * faster.  chosen (nullable) receives up to nchosen values: scat_min, zchunk,
+ * cls_rows, slab, zauto; where the automatic column length beats every fixed
+ * one it stays in force (zauto 1) and zchunk is the fastest fixed one.
  */
 int tam_autotune(struct tam_ctx *ctx, int64_t packets, int32_t steps, int64_t *chosen, int32_t nchosen);
 /* Autotuner of the batched heat step: times `steps` batched steps of the n

@@ -198,10 +198,12 @@ class Context:
         self._ck(self._lib.tam_load_state(self._h, str(path).encode()))
 
     def autotune(self, packets: int = 1_000_000, steps: int = 20) -> dict:
-        """Pick the fastest kernel settings on this context's workload; state is restored."""
-        out = (C.c_int64 * 4)()
-        self._ck(self._lib.tam_autotune(self._h, int(packets), int(steps), out, 4))
-        return {"transport.scat_min": out[0], "heat.zchunk": out[1], "heat.cls_rows": out[2], "heat.slab": out[3]}
+        """Pick the fastest kernel settings on this context's workload; state is restored.
+        Returns the settings now in force, in an order in which `set_tuning` can repeat them."""
+        out = (C.c_int64 * 5)()
+        self._ck(self._lib.tam_autotune(self._h, int(packets), int(steps), out, 5))
+        return {"transport.scat_min": out[0], "heat.zchunk": out[1], "heat.cls_rows": out[2], "heat.slab": out[3],
+                "heat.zauto": out[4]}
 
     def write_output(self, directory: str) -> None:
         self._ck(self._lib.tam_write_output(self._h, directory.encode()))
