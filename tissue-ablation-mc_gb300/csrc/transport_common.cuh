@@ -43,7 +43,8 @@ __device__ __forceinline__ double div64(double a, double b)
 }
 // |n| below 1e-289, where the reciprocal leaves the normal numbers
 __device__ __forceinline__ bool is_tiny(double n) { return (__double2hiint(n) & 0x7fffffff) < 0x03e00000; }
-// Square root of a normal operand or zero: g -> sqrt(x) and h -> 1 / (2 sqrt(x)) together
+// Square root of a normal operand or zero (a subnormal one, whose root is below 1e-153,
+// is returned as it is): g -> sqrt(x) and h -> 1 / (2 sqrt(x)) together
 // from the hardware's approximation (Goldschmidt), then one correction by the remainder
 // (Markstein): 7 operations, the bits of the IEEE square root for all of 2e8 operands.
 __device__ __forceinline__ double sqrt64(double x)
@@ -55,7 +56,7 @@ __device__ __forceinline__ double sqrt64(double x)
     g = __fma_rn(g, r, g);
     h = __fma_rn(h, r, h);
     g = __fma_rn(__fma_rn(-g, g, x), h, g);
-    return ieee::is_zero(x) ? x : g;
+    return (__double2hiint(x) & 0x7fffffff) < 0x00100000 ? x : g;
 }
 // |a| > 1, |a| < 1 and the sign, off the FP64 pipe (a NaN counts as neither)
 __device__ __forceinline__ bool above_one(double a) { return (ieee::bits(a) & ~ieee::SIGN) - (ieee::ONE + 1) < ieee::PINF - ieee::ONE; }
