@@ -160,6 +160,10 @@ __device__ __forceinline__ void ghost4(const FusedArgs &a, int f, const float4 &
 struct QConst {
     float2 Cx, Cy, Cz, C6, Ku;
 };
+// Two voxels' coefficients, face by face.
+struct Coef {
+    float2 zm, zp, ym, yp, xm, xp, Ku;
+};
 __device__ __forceinline__ QConst qconst(const FusedArgs &a, float au, float irc, float Pdt)
 {
     const float x = a.fc[FC_DT] * a.fc[FC_CX] * au, y = a.fc[FC_DT] * a.fc[FC_CY] * au, z = a.fc[FC_DT] * a.fc[FC_CZ] * au;
@@ -180,10 +184,11 @@ constexpr int QS_FACES = 16;  // status c + QS_FACES: class c throughout, summed
 // class c: the face-by-face sum of a grid of several classes, with one
 // coefficient per axis; 0xFF: a coefficient per face.
 __global__ void quad_status_kernel(const uint8_t *cls, int pitch, int nx, int ny, int nz, const uint8_t *bclass, int tx,
-                                   int ty, int zc, uint8_t *qs)
+                                   int ty, int zc, uint8_t *qs, unsigned *nmixed)
 {
     const int nq = nx / 4, nzc = (nz + zc - 1) / zc;
     const int64_t n = (int64_t)nq * ny * nz;
+    unsigned mixed = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int x = 4 * (int)(i % nq), y = (int)(i / nq % ny), z = (int)(i / nq / ny);
         const int bc = bclass[((int64_t)(nzc - 1 - z / zc) * ty + y / TR) * tx + x / TW];
@@ -205,27 +210,61 @@ __global__ void quad_status_kernel(const uint8_t *cls, int pitch, int nx, int ny
         if (z > 0) look(p - (int64_t)pitch * ny, 4);
         if (z + 1 < nz) look(p + (int64_t)pitch * ny, 4);
         qs[i] = (uint8_t)(one ? c + QS_FACES : 0xFF);
+        mixed += one ? 0u : 1u;
     }
+    mixed = __reduce_add_sync(0xffffffffu, mixed);
+    if ((threadIdx.x & 31) == 0 && mixed) atomicAdd(nmixed, mixed);
 }
 
-template <bool HET>
-__global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
+// The kernel's forms: a grid of one class; of several, the quads beside another class
+// listed and taken at the block's end; the same with those quads done in their plane.
+//
+// Listed, the quads beside another class cost a pass of scattered loads: on grids full of
+// class boundaries that was most of the step (192^3 of random classes 113 us, of 8^3
+// blocks 95, where the staged form took 47).  In their plane each voxel looks up its
+// classes, a word per quad and neighbour (the next plane's is carried on, and so are the
+// coefficients of the faces above), and its coefficients in shared memory: 44.5 and 44.4
+// us, with the listed form's operations and bits.  5 blocks per SM at 96 registers, no
+// spills (6 at 80: 192^3 46.0, 256^3 85.5 -> 95.8).
+enum QForm { Q_ONE, Q_LISTED, Q_MIXED };
+// Q_MIXED from this share of quads beside another class.  us per step listed / in the
+// plane: 256^3 2 % 77.5 / 88.4, 9 % 104 / 91, 21 % 121 / 88; 192^3 2 % 37.4 / 44.3, 9 %
+// 49.7 / 46.3; 128^3 2 % 14.0 / 15.7, 7 % 18.2 / 16.0; 256 x 256 x 128 in three layers
+// (3 %) 54.7 / 57.6, 96 x 96 x 48 (8 %) 12.1 / 7.7.  (One quad in twelve beside another
+// class is the worst of both: the staged form took 43.1 us there on 192^3, 90.1 on 256^3.)
+constexpr int QMIX_SHARE = 20;
+
+template <int FORM>
+__global__ void __launch_bounds__(QTPB, FORM == Q_ONE ? 8 : (FORM == Q_LISTED ? 7 : 5))
     quad_step_kernel(const __grid_constant__ FusedArgs a, const __grid_constant__ ClassLut L,
                      const __grid_constant__ QClasses C, int zchunk, float rare_thr)
 {
+    constexpr bool HET = FORM != Q_ONE, MIX = FORM == Q_MIXED;
     __shared__ unsigned short s_list[QTPB * 4 * QZMAX];
     __shared__ int s_cnt;
-    __shared__ unsigned short s_faces[HET ? QTPB * QZMAX : 1];
+    __shared__ unsigned short s_faces[FORM == Q_LISTED ? QTPB * QZMAX : 1];
     __shared__ int s_nf;
-    __shared__ float s_fa[HET ? MAX_MAT * MAX_MAT : 1];
+    // face coefficients (MIX: times the axis's factor, x, y, z)
+    __shared__ float s_fa[HET ? (MIX ? 3 : 1) * MAX_MAT * MAX_MAT : 1];
     __shared__ QConst s_q[HET ? MAX_MAT : 1];
+    __shared__ float s_k[MIX ? MAX_MAT : 1];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) s_cnt = s_nf = 0;
     const float Pdt = step_pdt<float>(a);
     const bool src = Pdt != 0.f;  // without a source J is not read
     if (HET) {
         constexpr int N = MAX_MAT * MAX_MAT;
-        for (int t = threadIdx.x; t < N; t += QTPB) s_fa[t] = __ldg(C.tab + t);
+        for (int t = threadIdx.x; t < N; t += QTPB) {
+            const float f = __ldg(C.tab + t);
+            if (MIX) {
+                s_fa[t] = a.fc[FC_DT] * a.fc[FC_CX] * f;
+                s_fa[N + t] = a.fc[FC_DT] * a.fc[FC_CY] * f;
+                s_fa[2 * N + t] = a.fc[FC_DT] * a.fc[FC_CZ] * f;
+            } else {
+                s_fa[t] = f;
+            }
+        }
+        if (MIX && threadIdx.x < MAX_MAT) s_k[threadIdx.x] = L.k[threadIdx.x];
         if (threadIdx.x < MAX_MAT) s_q[threadIdx.x] = qconst(a, __ldg(C.tab + threadIdx.x * (MAX_MAT + 1)), __ldg(C.tab + N + threadIdx.x), Pdt);
     }
     __syncthreads();
@@ -254,6 +293,24 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
         const QConst qu = qconst(a, L.fa[uc * MAX_MAT + uc], L.irc[uc], Pdt);
         const QConst *qp = &qu;
         int st = 0;  // HET: the quad's status
+        // MIX: the classes of the quad's voxels and of those in the planes around it, a byte each
+        constexpr unsigned CMASK = 0x01010101u * (MAX_MAT - 1);
+        const int64_t cpl = (int64_t)C.cpitch * ny;
+        const uint8_t *cp = MIX ? C.cls + (act ? x + (int64_t)C.cpitch * y : 0) + cpl * z0 : nullptr;
+        const int cyl = oyl ? -C.cpitch : 0, cyh = oyh ? C.cpitch : 0;
+        auto word = [](const uint8_t *p) { return __ldg(reinterpret_cast<const unsigned *>(p)) & CMASK; };
+        // entry of the face table: byte b of a word of index pairs
+        auto fa = [&](int axis, unsigned w, int b) {
+            const unsigned o = (b ? w >> (8 * b - 2) : w << 2) & 0x3FCu;
+            return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(s_fa + axis * MAX_MAT * MAX_MAT) + o);
+        };
+        unsigned kc = 0;
+        float4 fzc = make_float4(0.f, 0.f, 0.f, 0.f);  // coefficients of the faces below
+        if (MIX) {
+            kc = word(cp);
+            const unsigned w = kc << 4 | (z0 > 0 ? word(cp - cpl) : kc);
+            fzc = make_float4(fa(2, w, 0), fa(2, w, 1), fa(2, w, 2), fa(2, w, 3));
+        }
         float4 A[3], B[3];  // T and the Kahan term of three planes, in rotation
         {
             const int w = v - (z0 > 0 ? pl : 0);
@@ -278,9 +335,43 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
                 st = __ldg(C.qs + (v >> 2));
                 qp = s_q + (st & (QS_FACES - 1));
             }
+            unsigned kn = 0, kyl = 0, kyh = 0, kxl = 0, kxr = 0;
+            if (MIX) {
+                // (outside the grid: the voxel's own class)
+                kn = z + 1 < nz ? word(cp + cpl) : kc;
+                kyl = word(cp + cyl), kyh = word(cp + cyh);
+                const unsigned ke = ed ? __ldg(cp + oe) & (MAX_MAT - 1) : 0u;
+                kxl = __shfl_up_sync(0xffffffffu, kc, 1) >> 24, kxr = __shfl_down_sync(0xffffffffu, kc, 1) & (MAX_MAT - 1);
+                if (lane == 0) kxl = ke;
+                if (lane == 31) kxr = ke;
+                if (x == 0) kxl = kc & (MAX_MAT - 1);
+                if (x + 4 == nx) kxr = kc >> 24;
+            }
+            // the next plane's faces below are this plane's faces above
+            float4 fzn = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (MIX) {
+                const unsigned w = kc << 4 | kn;
+                fzn = make_float4(fa(2, w, 0), fa(2, w, 1), fa(2, w, 2), fa(2, w, 3));
+            }
             const QConst &q = *qp;
             float4 tn = tnx, en = enx;
-            if (bnd) {
+            if (MIX) {
+                // ghost neighbours, each voxel of its own class
+                auto ghosts = [&](int f, float4 &t, float4 &e) {
+                    ghost1<true>(a, f, tc.x, ec.x, s_k[kc & 255u], t.x, e.x);
+                    ghost1<true>(a, f, tc.y, ec.y, s_k[kc >> 8 & 255u], t.y, e.y);
+                    ghost1<true>(a, f, tc.z, ec.z, s_k[kc >> 16 & 255u], t.z, e.z);
+                    ghost1<true>(a, f, tc.w, ec.w, s_k[kc >> 24], t.w, e.w);
+                };
+                if (bnd) {
+                    if (x == 0) ghost1<true>(a, 0, tc.x, ec.x, s_k[kc & 255u], xl, el);
+                    if (x + 4 == nx) ghost1<true>(a, 1, tc.w, ec.w, s_k[kc >> 24], xr, er);
+                    if (y == 0) ghosts(2, yl, yel);
+                    if (y == ny - 1) ghosts(3, yh, yeh);
+                }
+                if (z == 0) ghosts(4, tp, ep);
+                if (z == nz - 1) ghosts(5, tn, en);
+            } else if (bnd) {
                 // ghost neighbours
                 const float k = L.k[HET ? st & (QS_FACES - 1) : uc];
                 if (x == 0) ghost1<false>(a, 0, tc.x, ec.x, k, xl, el);
@@ -288,8 +379,8 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
                 if (y == 0) ghost4<HET>(a, 2, tc, ec, k, yl, yel);
                 if (y == ny - 1) ghost4<HET>(a, 3, tc, ec, k, yh, yeh);
             }
-            if (z == 0) ghost4<HET>(a, 4, tc, ec, L.k[HET ? st & (QS_FACES - 1) : uc], tp, ep);
-            if (z == nz - 1) ghost4<HET>(a, 5, tc, ec, L.k[HET ? st & (QS_FACES - 1) : uc], tn, en);
+            if (!MIX && z == 0) ghost4<HET>(a, 4, tc, ec, L.k[HET ? st & (QS_FACES - 1) : uc], tp, ep);
+            if (!MIX && z == nz - 1) ghost4<HET>(a, 5, tc, ec, L.k[HET ? st & (QS_FACES - 1) : uc], tn, en);
             float2 t0 = {}, e0 = {}, t1 = {}, e1 = {};
             if (!HET || st < QS_FACES) {
                 // sum over the faces of C_f [(T_f - T_c) - (e_f - e_c)]; x: face differences once each
@@ -307,28 +398,38 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
                 };
                 half(lo2(tc), lo2(ec), sx0, lo2(yl), lo2(yh), lo2(yel), lo2(yeh), lo2(tp), lo2(tn), lo2(ep), lo2(en), lo2(j), t0, e0);
                 half(hi2(tc), hi2(ec), sx1, hi2(yl), hi2(yh), hi2(yel), hi2(yeh), hi2(tp), hi2(tn), hi2(ep), hi2(en), hi2(j), t1, e1);
-            } else if (st < 2 * QS_FACES) {
-                // one class around: face by face, as beside other classes
+            } else if (MIX || st < 2 * QS_FACES) {
+                // face by face; one class around: with one coefficient per axis
                 const float dx0 = (xl - tc.x) - (el - ec.x), dx1 = (tc.y - tc.x) - (ec.y - ec.x);
                 const float dx2 = (tc.z - tc.y) - (ec.z - ec.y), dx3 = (tc.w - tc.z) - (ec.w - ec.z);
                 const float dx4 = (xr - tc.w) - (er - ec.w);
                 auto half = [&](float2 c, float2 e, float2 xm, float2 xp, float2 ym, float2 yp, float2 em, float2 eq,
-                                float2 zm, float2 zp, float2 fm, float2 fq, float2 jj, float2 &tt, float2 &ek) {
+                                float2 zm, float2 zp, float2 fm, float2 fq, float2 jj, const Coef &F, float2 &tt, float2 &ek) {
                     const float2 zM = sub2(sub2(zm, c), sub2(fm, e)), zP = sub2(sub2(zp, c), sub2(fq, e));
                     const float2 yM = sub2(sub2(ym, c), sub2(em, e)), yP = sub2(sub2(yp, c), sub2(eq, e));
-                    const float2 cx = q.Cx, cy = q.Cy, cz = q.Cz;
-                    const float2 dT = add2(add2(fma2(cz, zM, mul2(cz, zP)), fma2(cy, yM, mul2(cy, yP))), fma2(cx, xm, mul2(cx, xp)));
-                    const float2 yk = sub2(fma2(q.Ku, jj, dT), e);
+                    const float2 dT = add2(add2(fma2(F.zm, zM, mul2(F.zp, zP)), fma2(F.ym, yM, mul2(F.yp, yP))), fma2(F.xm, xm, mul2(F.xp, xp)));
+                    const float2 yk = sub2(fma2(F.Ku, jj, dT), e);
                     tt = add2(c, yk);
                     ek = sub2(sub2(tt, c), yk);
                 };
-                half(lo2(tc), lo2(ec), make_float2(dx0, -dx1), make_float2(dx1, dx2), lo2(yl), lo2(yh), lo2(yel), lo2(yeh), lo2(tp), lo2(tn), lo2(ep), lo2(en), lo2(j), t0, e0);
-                half(hi2(tc), hi2(ec), make_float2(-dx2, -dx3), make_float2(dx3, dx4), hi2(yl), hi2(yh), hi2(yel), hi2(yeh), hi2(tp), hi2(tn), hi2(ep), hi2(en), hi2(j), t1, e1);
+                // the coefficients of voxels b and b + 1 of the quad; pairs of classes, own and neighbour's
+                const unsigned own = kc << 4;
+                auto coef = [&](int b) -> Coef {
+                    if (!MIX) return Coef{q.Cz, q.Cz, q.Cy, q.Cy, q.Cx, q.Cx, q.Ku};
+                    auto two = [&](int axis, unsigned w) { return make_float2(fa(axis, w, b), fa(axis, w, b + 1)); };
+                    const unsigned wx = own | kc >> 8;  // with the next voxel of the quad
+                    const float mid = fa(0, wx, b);
+                    const float2 xm = make_float2(b ? fa(0, wx, 1) : fa(0, own | kxl, 0), mid), xp = make_float2(mid, b ? fa(0, own >> 24 | kxr, 0) : fa(0, wx, 1));
+                    auto ku = [&](int i) { return s_q[kc >> (8 * i) & 255u].Ku.x; };
+                    return Coef{b ? hi2(fzc) : lo2(fzc), b ? hi2(fzn) : lo2(fzn), two(1, own | kyl), two(1, own | kyh), xm, xp, make_float2(ku(b), ku(b + 1))};
+                };
+                half(lo2(tc), lo2(ec), make_float2(dx0, -dx1), make_float2(dx1, dx2), lo2(yl), lo2(yh), lo2(yel), lo2(yeh), lo2(tp), lo2(tn), lo2(ep), lo2(en), lo2(j), coef(0), t0, e0);
+                half(hi2(tc), hi2(ec), make_float2(-dx2, -dx3), make_float2(dx3, dx4), hi2(yl), hi2(yh), hi2(yel), hi2(yeh), hi2(tp), hi2(tn), hi2(ep), hi2(en), hi2(j), coef(2), t1, e1);
             } else if (act) {
                 // several classes around: after the planes, see below
                 s_faces[atomicAdd(&s_nf, 1)] = (unsigned short)((z - z0) * QTPB + (int)threadIdx.x);
             }
-            if (act && (!HET || st != 0xFF)) {
+            if (act && (FORM != Q_LISTED || st != 0xFF)) {
                 *reinterpret_cast<float4 *>(To + v) = make_float4(t0.x, t0.y, t1.x, t1.y);
                 *reinterpret_cast<float4 *>(Eo + v) = make_float4(e0.x, e0.y, e1.x, e1.y);
                 // listed: an old or new temperature at the screen, negative or NaN
@@ -346,6 +447,7 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
                 }
             }
             v += pl;
+            if (MIX) kc = kn, fzc = fzn, cp += act ? cpl : 0;
         };
         for (int z = z0;;) {
             step(z, A[0], B[0], A[1], B[1], A[2], B[2]);
@@ -357,7 +459,7 @@ __global__ void __launch_bounds__(QTPB, HET ? 7 : 8)
         }
     }
     __syncthreads();
-    if (HET) {
+    if (FORM == Q_LISTED) {
         // Voxels beside another class, a coefficient per face, one per thread: few lie
         // together (2.6 quads in each of 24 % of the warps on 256^3 vessels), and
         // inside the planes each holds up its warp (142 us per step against 78).  A
@@ -445,17 +547,19 @@ bool quad_step_supported(int nx, int ny, int nz)
 
 static int64_t tiles_of(int nx, int ny, int nz) { return (int64_t)((nx + TW - 1) / TW) * ((ny + TR - 1) / TR) * nz; }
 
-constexpr int64_t TAB_BYTES = 4 * MAX_MAT * (MAX_MAT + 1);
+// face table, 1 / (rho c), the count of quads beside another class
+constexpr int64_t CNT_AT = 4 * MAX_MAT * (MAX_MAT + 1), TAB_BYTES = CNT_AT + 16;
 
 int64_t quad_class_bytes(int nx, int ny, int nz) { return TAB_BYTES + (int64_t)(nx / 4) * ny * nz + 2 * tiles_of(nx, ny, nz); }
 
 cudaError_t launch_quad_classes(const ClassLut &L, const uint8_t *cls, int pitch, int nx, int ny, int nz, int zchunk, uint8_t *mem,
-                                cudaStream_t s)
+                                bool *mixed, cudaStream_t s)
 {
-    float tab[MAX_MAT * (MAX_MAT + 1)];
+    float tab[MAX_MAT * (MAX_MAT + 1) + 1];
     std::memcpy(tab, L.fa, 4 * MAX_MAT * MAX_MAT);
     std::memcpy(tab + MAX_MAT * MAX_MAT, L.irc, 4 * MAX_MAT);
-    const cudaError_t e = cudaMemcpyAsync(mem, tab, sizeof tab, cudaMemcpyHostToDevice, s);
+    tab[MAX_MAT * (MAX_MAT + 1)] = 0.f;  // the count
+    cudaError_t e = cudaMemcpyAsync(mem, tab, sizeof tab, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return e;
     uint8_t *qs = mem + TAB_BYTES;
     // the runs that one-class tiles are looked for in
@@ -467,12 +571,16 @@ cudaError_t launch_quad_classes(const ClassLut &L, const uint8_t *cls, int pitch
     count_launch(3);
     tile_flags_kernel<<<blocks(tiles, 8), 256, 0, s>>>(cls, pitch, nx, ny, nz, tflag);
     block_class_kernel<<<blocks(items, 256), 256, 0, s>>>(tflag, tx, ty, nz, zc, bclass);
-    quad_status_kernel<<<blocks(quads, 256), 256, 0, s>>>(cls, pitch, nx, ny, nz, bclass, tx, ty, zc, qs);
-    return cudaGetLastError();
+    quad_status_kernel<<<blocks(quads, 256), 256, 0, s>>>(cls, pitch, nx, ny, nz, bclass, tx, ty, zc, qs, (unsigned *)(mem + CNT_AT));
+    unsigned n = 0;
+    if ((e = cudaGetLastError()) == cudaSuccess) e = cudaMemcpyAsync(&n, mem + CNT_AT, sizeof n, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    *mixed = (int64_t)n * QMIX_SHARE > quads;
+    return e;
 }
 
 cudaError_t launch_quad_step(const FusedArgs &a0, const ClassLut &L, const uint8_t *cls, int cpitch, const uint8_t *mem,
-                             cudaStream_t s)
+                             bool mixed, cudaStream_t s)
 {
     FusedArgs a = a0;
     fill_fused_consts(a);
@@ -495,8 +603,9 @@ cudaError_t launch_quad_step(const FusedArgs &a0, const ClassLut &L, const uint8
     cfg.attrs = at;
     cfg.numAttrs = 1;
     count_launch();
-    return L.uniform >= 0 ? cudaLaunchKernelEx(&cfg, quad_step_kernel<false>, a, L, C, zc, rare_thr)
-                          : cudaLaunchKernelEx(&cfg, quad_step_kernel<true>, a, L, C, zc, rare_thr);
+    if (L.uniform >= 0) return cudaLaunchKernelEx(&cfg, quad_step_kernel<Q_ONE>, a, L, C, zc, rare_thr);
+    return mixed ? cudaLaunchKernelEx(&cfg, quad_step_kernel<Q_MIXED>, a, L, C, zc, rare_thr)
+                 : cudaLaunchKernelEx(&cfg, quad_step_kernel<Q_LISTED>, a, L, C, zc, rare_thr);
 }
 
 }  // namespace tam

@@ -155,7 +155,7 @@ struct tam_ctx {
     // grid, made when a heat call finds it out of date
     bool quad = false;
     uint8_t *d_qs = nullptr;
-    bool qs_ok = false;
+    bool qs_ok = false, qs_mixed = false;
     bool use_slab = true;            // class-table step: the quad form where the grid allows it
     uint8_t *d_cls = nullptr;
     int cls_pitch = 0;
@@ -976,7 +976,7 @@ int quad_classes(tam_ctx *ctx)
         return TAM_OK;
     }
     CK(tam::launch_quad_classes(ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->nx, ctx->ny, ctx->nz, zchunk_of(ctx), ctx->d_qs,
-                                ctx->stream));
+                                &ctx->qs_mixed, ctx->stream));
     ctx->qs_ok = true;
     return TAM_OK;
 }
@@ -1019,7 +1019,7 @@ int launch_heat(tam_ctx *ctx, tam::FusedArgs &a, HeatForm form, int which, cudaS
     a.Tc_in = ctx->fp64 ? nullptr : ctx->d_Tc[which];
     a.Tc_out = ctx->fp64 ? nullptr : ctx->d_Tc[1 - which];
     switch (form) {
-    case HF_QUAD: CK(tam::launch_quad_step(a, ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->d_qs, s)); break;
+    case HF_QUAD: CK(tam::launch_quad_step(a, ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->d_qs, ctx->qs_mixed, s)); break;
     case HF_CLS: CK(tam::launch_fused_cls(a, ctx->fcls, which, ctx->clut, ctx->cls_rows, s)); break;
     case HF_LINE: CK(tam::launch_line_step(a, ctx->clut, ctx->d_cls, ctx->cls_pitch, ctx->d_ltab, s)); break;
     case HF_TMA: CK(tam::launch_fused_tma(a, ctx->tma, which, s)); break;
@@ -1045,7 +1045,7 @@ std::vector<unsigned char> graph_key(const tam_ctx *ctx, const tam::FusedArgs &a
     a.T_in = a.T_out = nullptr;
     a.Tc_in = nullptr;
     a.Tc_out = nullptr;
-    const int knobs[4] = {(int)form, ctx->cls_rows, zchunk_of(ctx), ctx->arr_fp64 ? 1 : 0};
+    const int knobs[5] = {(int)form, ctx->cls_rows, zchunk_of(ctx), ctx->arr_fp64 ? 1 : 0, ctx->qs_mixed ? 1 : 0};
     std::vector<unsigned char> k(sizeof a + sizeof ctx->clut + sizeof knobs + 2 * sizeof(void *));
     unsigned char *p = k.data();
     std::memcpy(p, &a, sizeof a);

@@ -364,10 +364,11 @@ bool quad_step_supported(int nx, int ny, int nz);
 // Heterogeneous grids: the update that each quad's classes ask for.  Where a 32 x 8
 // tile, its x / y rim and a run of planes (heat.zchunk of them, 6 by default, at
 // most 8, and the planes beside them) hold one class, that is the one-class
-// update.  qs: quad_class_bytes.
+// update.  qs: quad_class_bytes.  *mixed: whether so many quads lie beside another
+// class that the step takes them in their planes (read back: synchronises the stream).
 int64_t quad_class_bytes(int nx, int ny, int nz);
 cudaError_t launch_quad_classes(const ClassLut &L, const uint8_t *cls, int pitch, int nx, int ny, int nz, int zchunk,
-                                uint8_t *qs, cudaStream_t s);
+                                uint8_t *qs, bool *mixed, cudaStream_t s);
 // Line form (heat_line.cu): rows of any width, fewer than 2^31 voxels.  tab:
 // LINE_TABLE floats, the face table of a heterogeneous grid.
 constexpr int LINE_TABLE = MAX_MAT * MAX_MAT;
@@ -377,7 +378,7 @@ cudaError_t launch_line_step(const FusedArgs &a, const ClassLut &L, const uint8_
                              cudaStream_t s);
 // One step, as a programmatic dependent of the launch before it.
 cudaError_t launch_quad_step(const FusedArgs &a, const ClassLut &L, const uint8_t *cls, int cpitch, const uint8_t *qs,
-                             cudaStream_t s);
+                             bool mixed, cudaStream_t s);
 
 // Batched FP32 heat step of many instances in one persistent cooperative
 // launch (batch.cu).  BatchInst lives in device memory, one per instance.
