@@ -136,10 +136,12 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     // per-packet (rare) tallies accumulate in shared memory, not registers
     __shared__ double s_tal[5];  // specular, reflected, transmitted, side, roulette net
     __shared__ unsigned long long s_cnt[2];  // voxel steps, scatters
+    __shared__ unsigned s_entered[MAX_MAT];  // packets launched into each material (FP32)
     __shared__ unsigned s_err;
     constexpr bool SCAT64 = sizeof(Real) == 8 && MED != MED_RHOKAP;  // the reference medium only absorbs
     if (threadIdx.x < 5) s_tal[threadIdx.x] = 0.0;
     if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
+    if (threadIdx.x < MAX_MAT) s_entered[threadIdx.x] = 0u;
     if (threadIdx.x == 0) s_err = 0u;
     __syncthreads();
 
@@ -183,9 +185,11 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     Real w = 0, tau = 0, dep = 0, mut = 0, mua = 0;
     uint32_t ev = 0, plo = 0, phi32 = 0, nsteps = 0;
     uint32_t cScat = 0;
-    // The specular tally: FP64 additions to one shared word go lane by lane, 32 of them
-    // whenever a warp launches together, and a packet of the reference medium does
-    // little else.  (FP32: the sum costs more than the contention, 0.8 us per pass.)
+    // The specular tally: FP64 additions to one shared word go lane by lane, a compare
+    // and swap each, 32 of them whenever a warp launches together, which packets that
+    // end after a few steps do often.  So FP64 sums in a register, and FP32, short of
+    // registers, counts the packets that entered each material, one instruction for the
+    // warp (2e6 packets, 128^3, mua 50 / mus 10 per cm: 939 -> 697 us).
     constexpr bool SPEC_REG = sizeof(Real) == 8;
     double spec = 0.0;
     uint64_t cSteps = 0;  // voxel steps of this thread's finished packets (reduced once at the end)
@@ -275,7 +279,7 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
                                 rsp = rsp * rsp;
                             }
                             if constexpr (SPEC_REG) spec += (double)rsp;
-                            else atomicAdd(&s_tal[0], (double)rsp);
+                            else atomicAdd(&s_entered[MED == MED_MATERIAL ? mid : 0], 1u);
                             w = (Real)1 - rsp;
                         }
                         tau = M<Real>::neglog(u3);
@@ -587,6 +591,13 @@ __global__ void __launch_bounds__(TPB, sizeof(Real) == 4 ? TAM_TR_MINB : 2) tran
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        if (!SPEC_REG && a.fresnel) {
+            for (int m = 0; m < (MED == MED_MATERIAL ? a.nmat : 1); ++m) {
+                const Real nt = MED == MED_RHOKAP ? K.rhokap_n : lut[MED == MED_MATERIAL ? m : mid_u].n;
+                const Real r = (namb - nt) / (namb + nt);
+                s_tal[0] += (double)s_entered[m] * (double)(r * r);
+            }
+        }
         atomicAdd(a.tally + T_SPECULAR, s_tal[0]);
         atomicAdd(a.tally + T_REFLECTED, s_tal[1]);
         atomicAdd(a.tally + T_TRANSMITTED, s_tal[2]);
