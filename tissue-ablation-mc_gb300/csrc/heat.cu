@@ -211,6 +211,12 @@ __global__ void __launch_bounds__(REF_TPB, REF_BLOCKS) ref_stencil_kernel(const 
     using O = RefOps<F>;
     constexpr int R = REF_ROWS;
     constexpr bool D = sizeof(F) == 8;
+    // A coefficient that two of the thread's voxels share is formed once: in FP64 only in
+    // steps of their own, where a caller's per-voxel properties leave no cell a class (80^3
+    // 112.6 -> 96.3 us, 128^3 415 -> 350; every coefficient twice was slower there than the
+    // kernel of three divisions a voxel, 104 and 378).  In the loop few cells have none, and
+    // the registers cost more than it saves (68.5 -> 68.8 us per iteration).
+    constexpr bool SHARE = !D || !RAW;
     const RefHeatArgs &a = a0;
     // the iteration's laserOn from device memory when replayed from a graph
     const double laserOn = a.laser_dev ? *a.laser_dev : a.laserOn;
@@ -268,7 +274,8 @@ __global__ void __launch_bounds__(REF_TPB, REF_BLOCKS) ref_stencil_kernel(const 
     F tm[R], t[R];
     int km[R], kc[R];
     double pm[R], p0[R];  // D: g T of the plane below and of this one
-    F fz[R];              // else: the coefficient of the face below
+    F fz[R];              // else, and with zg: the coefficient of the face below
+    bool zg = false;      // SHARE: the plane below took its coefficients (the whole warp)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         tm[r] = tt[c[r] - sz];
@@ -311,15 +318,19 @@ __global__ void __launch_bounds__(REF_TPB, REF_BLOCKS) ref_stencil_kernel(const 
                 ys = ys && kc[r] == 0;
             }
             // whole warps of skin take the shared products
-            if (__all_sync(FULL, zs)) {
+            const bool zskin = __all_sync(FULL, zs);
+            if (zskin) {
 #pragma unroll
                 for (int r = 0; r < R; ++r) uz[r] = ADD(SUB(pm[r], ieee::twice_product(p0[r], gs[2], t[r])), pp[r]);
             } else {
 #pragma unroll
-                for (int r = 0; r < R; ++r)
-                    uz[r] = O::axis(face(km[r], kc[r], c[r] - sz, c[r], 2), face(kc[r], kp[r], c[r], c[r] + sz, 2), tm[r],
-                                    t[r], tp[r]);
+                for (int r = 0; r < R; ++r) {
+                    const F fzm = SHARE && zg ? fz[r] : face(km[r], kc[r], c[r] - sz, c[r], 2);
+                    fz[r] = face(kc[r], kp[r], c[r], c[r] + sz, 2);
+                    uz[r] = O::axis(fzm, fz[r], tm[r], t[r], tp[r]);
+                }
             }
+            if (SHARE) zg = !zskin;
             if (__all_sync(FULL, ys && in[R - 1])) {
                 double py[R + 2];
                 py[0] = MUL(gs[1], ym);
@@ -330,12 +341,16 @@ __global__ void __launch_bounds__(REF_TPB, REF_BLOCKS) ref_stencil_kernel(const 
                 for (int r = 0; r < R; ++r)
                     uy[r] = ADD(SUB(py[r], ieee::twice_product(py[r + 1], gs[1], t[r])), py[r + 2]);
             } else {
+                // (the face between the pair's rows once)
+                F fy = face(cym, kc[0], c[0] - sy, c[0], 1);
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const bool lo = r == 0, hi = r + 1 == R || !in[r + 1 < R ? r + 1 : r];
                     const F tl = lo ? ym : t[r > 0 ? r - 1 : 0], th = hi ? yp : t[r + 1 < R ? r + 1 : r];
-                    const int cl = lo ? cym : kc[r > 0 ? r - 1 : 0], ch = hi ? cyp : kc[r + 1 < R ? r + 1 : r];
-                    uy[r] = O::axis(face(cl, kc[r], c[r] - sy, c[r], 1), face(kc[r], ch, c[r], c[r] + sy, 1), tl, t[r], th);
+                    const int ch = hi ? cyp : kc[r + 1 < R ? r + 1 : r];
+                    const F fym = lo || SHARE ? fy : face(kc[0], kc[r], c[r] - sy, c[r], 1);
+                    fy = face(kc[r], ch, c[r], c[r] + sy, 1);
+                    uy[r] = O::axis(fym, fy, tl, t[r], th);
                 }
             }
 #pragma unroll
