@@ -69,6 +69,16 @@ struct __align__(16) BItem {
     int inst, x0, y0, z0, z1, cpitch;
 };
 
+// The ghosts of a pair across face f, written to its halo cells (out of line: rare).
+__device__ __noinline__ void y_ghosts(const FusedArgs &A, int f, float2 t, float2 e, float k0, float k1, float *WT, float *WE)
+{
+    const float2 g0 = ghost_pair(A, f, t.x, e.x, k0), g1 = ghost_pair(A, f, t.y, e.y, k1);
+    WT[0] = g0.x;
+    WT[1] = g1.x;
+    WE[0] = g0.y;
+    WE[1] = g1.y;
+}
+
 // The listed voxels of an item whose tile starts at (bxW, byR, zb) (the
 // block's own plane stores come first), as in the single-instance
 // kernel: the damage-window voxels' pairs and damage integrals loaded four
@@ -321,6 +331,13 @@ __global__ void __launch_bounds__(BP *BR, bslab_minb(UNIFORM))
                         WT[oS + 2] = g.x;
                         WE[oS + 2] = g.y;
                         if (!UNIFORM) WC[qC + 2] = (unsigned char)kc1;
+                    }
+                    if ((exy & 12u) == 12u) {  // one row in y: the same voxels' face above too
+                        y_ghosts(A, 3, Tc, Ec, L.k[kc0], L.k[kc1], WT + oP, WE + oP);
+                        if (!UNIFORM) {
+                            WC[qC + RC] = (unsigned char)kc0;
+                            WC[qC + 1 + RC] = (unsigned char)kc1;
+                        }
                     }
                     if (exy & 12u) {
                         const int f = (exy & 4u) ? 2 : 3, o = (exy & 4u) ? oM : oP, oc = (exy & 4u) ? -RC : RC;
@@ -677,6 +694,13 @@ __global__ void __launch_bounds__(BP *BR, UNIFORM ? TAM_BSTEP_MINB : 5)
                         WT[oS + 2] = g.x;
                         WE[oS + 2] = g.y;
                         if (!UNIFORM) WC[qC + 2] = (unsigned char)kc1;
+                    }
+                    if ((exy & 12u) == 12u) {  // one row in y: the same voxels' face above too
+                        y_ghosts(A, 3, Tc, Ec, L.k[kc0], L.k[kc1], WT + oP, WE + oP);
+                        if (!UNIFORM) {
+                            WC[qC + RC] = (unsigned char)kc0;
+                            WC[qC + 1 + RC] = (unsigned char)kc1;
+                        }
                     }
                     if (exy & 12u) {
                         const int f = (exy & 4u) ? 2 : 3, o = (exy & 4u) ? oM : oP, oc = (exy & 4u) ? -RC : RC;
