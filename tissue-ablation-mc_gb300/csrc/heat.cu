@@ -186,7 +186,7 @@ template <> struct RefOps<float> {
 // (FP64), 24 -> 15 us (FP32, which was bound by the latency of two barriers
 // per plane).  Threads take consecutive columns of the x-y plane, wrapping
 // from row pair to row pair, so no lane idles past a row's end.
-constexpr int REF_TPB = 128, REF_ROWS = 2, REF_BLOCKS = 6;  // blocks per SM: 80 registers (4: 2 to 6 % slower)
+constexpr int REF_TPB = 128, REF_ROWS = 2, REF_BLOCKS = 6;  // blocks per SM: 80 registers, in FP64 32 to 40 bytes spilled (4: 2 to 6 % slower)
 // a coefficient from the properties of its two cells (rare: kept out of line)
 template <typename F>
 __device__ __noinline__ F ref_face_at(const F *K, const F *Dn, const F *C, uint32_t p, uint32_t q, F id2)
@@ -599,8 +599,9 @@ __device__ __noinline__ void damage_props_voxel(const RefArrheniusArgs &d, const
 // that (the general path's compares took 360 instructions per warp; 80^3:
 // 14 -> 9.8 us).  Threads take consecutive cells of a plane, wrapping from row to
 // row.
-// (16 blocks of 128 threads per SM, 32 registers: the rare voxels' code takes 60 and
-// halved the warps that the calm ones' loads are in flight from.  Per iteration of the
+// (16 blocks of 128 threads per SM, 32 registers, 52 bytes spilled, and 76 in the rare
+// voxels' function: their code takes 60 and halved the warps that the calm ones' loads
+// are in flight from.  Per iteration of the
 // loop, before: 160^3 FP64 308 -> 290 us, FP32 164 -> 147; 80^3 76.1 -> 75.5)
 constexpr int PROPS_TPB = 128;
 __global__ void __launch_bounds__(PROPS_TPB, 16) ref_damage_props_kernel(const __grid_constant__ RefArrheniusArgs d,

@@ -7,8 +7,9 @@
 // differences along x formed once, and the rest of the arithmetic in two-wide
 // FP32 instructions (add / sub / fma.f32x2, each half rounded as the scalar
 // operation).  Latency is hidden by occupancy alone: 8 blocks of 128 threads per
-// SM at 64 registers; a plane of prefetch in registers cost two blocks per SM
-// and 15 % of the speed.  Threads take consecutive quads of a plane, wrapping from
+// SM at 64 registers (32 bytes spilled; several classes, listed: 7 at 72, 132 bytes;
+// in the plane: 5 at 96, none); a plane of prefetch in registers cost two blocks per
+// SM and 15 % of the speed.  Threads take consecutive quads of a plane, wrapping from
 // row to row, so that a block reads one run of memory (tiles 13 to 17 quads
 // wide: 20 % slower).
 //

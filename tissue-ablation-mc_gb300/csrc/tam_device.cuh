@@ -108,7 +108,6 @@ __device__ __forceinline__ double DIV(double a, double b) { return __ddiv_rn(a, 
 // ------------------------------------------------------- math dispatch --
 template <typename Real> struct M;
 template <> struct M<float> {
-    __device__ __forceinline__ static float log(float x) { return __logf(x); }
     // -log(u) for u in (0,1), never below 1 - u (> 0): the fast logarithm's
     // absolute error near 1 could otherwise give 0 or a negative value
     // (u is never subnormal: the flushing form of the logarithm)
@@ -120,19 +119,14 @@ template <> struct M<float> {
     }
     __device__ __forceinline__ static void sincos(float x, float *s, float *c) { __sincosf(x, s, c); }
     __device__ __forceinline__ static float sqrt(float x) { return sqrtf(x); }
-    __device__ __forceinline__ static float acos(float x) { return acosf(x); }
     __device__ __forceinline__ static float div(float a, float b) { return __fdividef(a, b); }
-    __device__ __forceinline__ static float rcp(float a) { return __frcp_rn(a); }  // correctly rounded 1/a
     __device__ __forceinline__ static float abs(float a) { return fabsf(a); }
 };
 template <> struct M<double> {
-    __device__ __forceinline__ static double log(double x) { return ::log(x); }
     __device__ __forceinline__ static double neglog(double u) { return -::log(u); }
     __device__ __forceinline__ static void sincos(double x, double *s, double *c) { ::sincos(x, s, c); }
     __device__ __forceinline__ static double sqrt(double x) { return ::sqrt(x); }
-    __device__ __forceinline__ static double acos(double x) { return ::acos(x); }
     __device__ __forceinline__ static double div(double a, double b) { return a / b; }
-    __device__ __forceinline__ static double rcp(double a) { return 1.0 / a; }
     __device__ __forceinline__ static double abs(double a) { return fabs(a); }
 };
 

@@ -19,6 +19,7 @@
 
 #include "tam_device.cuh"
 #include "tam_kernels.h"
+#include "scatter64.cuh"
 #include "transport_common.cuh"
 
 namespace tam {
