@@ -28,7 +28,7 @@
 // grid, 20 % of the time).  Per step with a core in the damage window, staged form
 // before -> now: 64^3 12.8 -> 5.9 us, 100^3 24.0 -> 7.0, 200^3 45.4 -> 30.6 (27.6
 // without a source), 256^3 70 -> 58.6, 384^3 218 -> 187; layers 96 x 96 x 48
-// 22.8 -> 11.4, 256 x 256 x 128 51.2 -> 50.0; vessels 96^3 21.6 -> 9.0, 256^3
+// 22.8 -> 6.9, 256 x 256 x 128 51.2 -> 49.3; vessels 96^3 21.6 -> 9.0, 256^3
 // 78.2 -> 77.6 (77.8 -> 71.8 without a source), 384^3 without a source 234 -> 214.
 #include <algorithm>
 #include <cstring>
